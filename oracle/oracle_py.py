@@ -335,7 +335,7 @@ def build(quiet: bool = True, ref: bool | None = None) -> None:
     targets = ["port", "opcount"]
     ref_src = reference_dir()
     if ref is None:
-        ref = ref_src.exists()
+        ref = (ref_src / "euler_equations").is_dir()
     if ref:
         targets.append("ref")
         if (HERE.parent / "cfd-art_b200" / "lib" / "libcfdgpu.so").exists():
