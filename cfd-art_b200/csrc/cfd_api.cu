@@ -90,9 +90,8 @@ namespace {
                         "%s: %s (%s:%d)", #expr, cudaGetErrorString(e_), __FILE__, __LINE__); \
     } while (0)
 
-// Tile shapes: x-sweep 64 cells along x by 4 rows; y-sweep 32 cells along y
-// by 8 columns.
-constexpr int TSX = 60, NAX = 4, TSY = 28, NAY = 8;
+constexpr int kSMs = 148;
+constexpr int kMaxCtas = 16 * kSMs;  // no sweep launches more
 
 int round_up(int v, int m) { return (v + m - 1) / m * m; }
 
@@ -169,9 +168,7 @@ Eos make_eos(const cfd_config& c) {
     q.p1 = c.pinf1;
     q.g2 = c.model == CFD_MODEL_ALLAIRE ? c.gamma2 : 1.4;
     q.p2 = c.model == CFD_MODEL_ALLAIRE ? c.pinf2 : 0.0;
-    q.gm1_1 = q.g1 - 1.0;
-    q.gm1_2 = q.g2 - 1.0;
-    q.gp1 = q.g1 * q.p1;
+    eos_derive(q);
     return q;
 }
 
@@ -191,31 +188,38 @@ void layout_sizes(const cfd_config& c, int& nv, int& g, int& pitch, long long& p
     buf_elems = (buf_elems + 31) / 32 * 32;
 }
 
-int sweep_blocks(const cfd_config& c, int dir) {
-    if (dir == DIR_X) return ((c.nx + TSX - 1) / TSX) * ((c.ny + NAX - 1) / NAX);
-    return ((c.ny + TSY - 1) / TSY) * ((c.nx + NAY - 1) / NAY);
+// Most CTAs of a sweep of either direction (the reduction's partials).
+int sweep_blocks(const cfd_config& c) {
+    const long long t = std::max(sweep_tiles<DIR_X>(c.nx, c.ny), sweep_tiles<DIR_Y>(c.nx, c.ny));
+    return (int)std::min<long long>(t, kMaxCtas);
 }
 
-template <int MODEL, int DIR, int TS, int NA>
-int launch_sweep_t(const SweepArgs& a, int blocks, cudaStream_t st) {
-    constexpr int smem = sweep_smem_bytes<MODEL, DIR, TS, NA>();
-    static bool attr_set = false;
-    if (!attr_set) {
-        CUDA_TRY(cudaFuncSetAttribute(sweep_kernel<MODEL, DIR, TS, NA>,
+// Persistent launch: as many CTAs as are resident at once, at most one per tile.
+template <int MODEL, int DIR>
+int launch_sweep_t(const SweepArgs& a, cudaStream_t st) {
+    constexpr int smem = sweep_smem_bytes<MODEL, DIR>();
+    static int per_sm = 0;
+    if (!per_sm) {
+        int n = 0;
+        CUDA_TRY(cudaFuncSetAttribute(sweep_kernel<MODEL, DIR>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        attr_set = true;
+        CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, sweep_kernel<MODEL, DIR>,
+                                                               sweep_threads<DIR>(), smem));
+        per_sm = std::max(1, std::min(n, kMaxCtas / kSMs));
     }
-    sweep_kernel<MODEL, DIR, TS, NA><<<blocks, 256, smem, st>>>(a);
+    const long long tiles = sweep_tiles<DIR>(a.nx, a.ny);
+    const int grid = (int)std::min<long long>(tiles, per_sm * kSMs);
+    sweep_kernel<MODEL, DIR><<<grid, sweep_threads<DIR>(), smem, st>>>(a);
     CUDA_TRY(cudaGetLastError());
     return CFD_OK;
 }
 
-int launch_sweep(int model, int dir, const SweepArgs& a, int blocks, cudaStream_t st) {
+int launch_sweep(int model, int dir, const SweepArgs& a, cudaStream_t st) {
     if (model == CFD_MODEL_EULER)
-        return dir == DIR_X ? launch_sweep_t<MODEL_EULER, DIR_X, TSX, NAX>(a, blocks, st)
-                            : launch_sweep_t<MODEL_EULER, DIR_Y, TSY, NAY>(a, blocks, st);
-    return dir == DIR_X ? launch_sweep_t<MODEL_ALLAIRE, DIR_X, TSX, NAX>(a, blocks, st)
-                        : launch_sweep_t<MODEL_ALLAIRE, DIR_Y, TSY, NAY>(a, blocks, st);
+        return dir == DIR_X ? launch_sweep_t<MODEL_EULER, DIR_X>(a, st)
+                            : launch_sweep_t<MODEL_EULER, DIR_Y>(a, st);
+    return dir == DIR_X ? launch_sweep_t<MODEL_ALLAIRE, DIR_X>(a, st)
+                        : launch_sweep_t<MODEL_ALLAIRE, DIR_Y>(a, st);
 }
 
 // Kernel arguments of one sweep reading bufs[cur ^ in_sel] and writing the
@@ -259,13 +263,13 @@ SweepArgs sweep_args(cfd_solver* s, int dir, int in_sel, double dt_scale, bool h
     return a;
 }
 
-int timed_sweep(cfd_solver* s, int dir, const SweepArgs& a, int blocks) {
-    if (!s->timing) return launch_sweep(s->cfg.model, dir, a, blocks, s->stream);
+int timed_sweep(cfd_solver* s, int dir, const SweepArgs& a) {
+    if (!s->timing) return launch_sweep(s->cfg.model, dir, a, s->stream);
     cudaEvent_t e0, e1;
     CUDA_TRY(cudaEventCreate(&e0));
     CUDA_TRY(cudaEventCreate(&e1));
     CUDA_TRY(cudaEventRecord(e0, s->stream));
-    int r = launch_sweep(s->cfg.model, dir, a, blocks, s->stream);
+    int r = launch_sweep(s->cfg.model, dir, a, s->stream);
     CUDA_TRY(cudaEventRecord(e1, s->stream));
     s->ev[dir].emplace_back(e0, e1);
     return r;
@@ -280,7 +284,6 @@ int enqueue_frame_snapshot(cfd_solver* s, int in_sel, bool host_dt);
 
 int enqueue_step(cfd_solver* s, bool host_dt, double dt) {
     const cfd_config& c = s->cfg;
-    int bx = sweep_blocks(c, DIR_X), by = sweep_blocks(c, DIR_Y);
     int r;
     // reference ghost values: the buffer current after the step keeps the
     // fill made before the sweep that read it last (naive: the x sweep;
@@ -288,17 +291,17 @@ int enqueue_step(cfd_solver* s, bool host_dt, double dt) {
     if (c.splitting == CFD_SPLIT_NAIVE) {
         if (s->ref_ghosts && (r = enqueue_frame_snapshot(s, 0, host_dt))) return r;
         SweepArgs ax = sweep_args(s, DIR_X, 0, 1.0, host_dt, dt, false, false);
-        if ((r = timed_sweep(s, DIR_X, ax, bx))) return r;
+        if ((r = timed_sweep(s, DIR_X, ax))) return r;
         SweepArgs ay = sweep_args(s, DIR_Y, 1, 1.0, host_dt, dt, true, false);
-        return timed_sweep(s, DIR_Y, ay, by);
+        return timed_sweep(s, DIR_Y, ay);
     }
     SweepArgs a1 = sweep_args(s, DIR_X, 0, 0.5, host_dt, dt, false, false);
-    if ((r = timed_sweep(s, DIR_X, a1, bx))) return r;
+    if ((r = timed_sweep(s, DIR_X, a1))) return r;
     if (s->ref_ghosts && (r = enqueue_frame_snapshot(s, 1, host_dt))) return r;
     SweepArgs a2 = sweep_args(s, DIR_Y, 1, 1.0, host_dt, dt, false, false);
-    if ((r = timed_sweep(s, DIR_Y, a2, by))) return r;
+    if ((r = timed_sweep(s, DIR_Y, a2))) return r;
     SweepArgs a3 = sweep_args(s, DIR_X, 0, 0.5, host_dt, dt, true, true);
-    return timed_sweep(s, DIR_X, a3, bx);
+    return timed_sweep(s, DIR_X, a3);
 }
 
 // ---- layout conversion and the initial reduction ---------------------------
@@ -553,76 +556,108 @@ __global__ void face_flux_kernel(int nfaces, const double* __restrict__ st, Eos 
     if (f >= nfaces) return;
     const int m = godunov ? 2 : 4;
     const double* S = st + (size_t)f * m * NV;
-    double EL[NV], ER[NV];
+    // the shared-reciprocal form, as in segment_update
+    Side<MODEL> L, R;
+    bool ok = true;
+    double F[NV], us, zL, zR;
     if (godunov) {
         for (int k = 0; k < NV; ++k) {
-            EL[k] = S[k];
-            ER[k] = S[NV + k];
+            L.U[k] = S[k];
+            R.U[k] = S[NV + k];
         }
+        ok &= side_from_cons<MODEL>(q, L);
+        ok &= side_from_cons<MODEL>(q, R);
     } else {
-        Prim<MODEL> P[4];
-        for (int c = 0; c < 4; ++c) cons_to_prim<MODEL>(q, S + c * NV, P[c]);
-        // cell 1 -> high-face states, cell 2 -> low-face states
-        double Ep[NV], Em[NV];
-        unsigned fl1 = 0, fl2 = 0;
+        PrimR<MODEL> P[4];
+        for (int c = 0; c < 4; ++c) ok &= c2p_rn<MODEL>(q, S + c * NV, P[c]);
         for (int side = 0; side < 2; ++side) {
-            int c = 1 + side;
-            double d[NV], Wt[NV], Ut[NV], e, X[NV];
+            const int c = 1 + side;  // cell 1 -> high-face state, cell 2 -> low-face state
+            double a[NV], b[NV], h[NV], Wt[NV], X[NV];
+            for (int k = 0; k < NV; ++k) {
+                a[k] = P[c].W[k] - P[c - 1].W[k];
+                b[k] = P[c + 1].W[k] - P[c].W[k];
+            }
+            limit_diffs<NV>(limiter, a, b, h);
+            ok &= jacobian_rn<MODEL>(q, P[c], h, s_half, X);
+            for (int k = 0; k < NV; ++k) h[k] = 0.5 * h[k];
+            ok &= slopes_physical<MODEL>(q, P[c].W, h);
             for (int k = 0; k < NV; ++k)
-                d[k] = limit1(limiter, P[c].W[k] - P[c - 1].W[k], P[c + 1].W[k] - P[c].W[k]);
-            unsigned fl = 0;
-            for (int k = 0; k < NV; ++k) Wt[k] = P[c].W[k] + 0.5 * d[k];
-            prim_to_cons<MODEL>(q, Wt, Ut, e);
-            if (muscl_check<MODEL>(Ut, Wt, e)) fl |= 1u;
-            for (int k = 0; k < NV; ++k) Wt[k] = P[c].W[k] - 0.5 * d[k];
-            prim_to_cons<MODEL>(q, Wt, Ut, e);
-            if (muscl_check<MODEL>(Ut, Wt, e)) fl |= 2u;
-            jacobian_times<MODEL>(q, P[c], d, s_half, X);
-            if (side == 0) {
-                for (int k = 0; k < NV; ++k) Wt[k] = (P[c].W[k] + 0.5 * d[k]) - X[k];
-                prim_to_cons<MODEL>(q, Wt, Ep, e);
-                if (muscl_check<MODEL>(Ep, Wt, e)) fl |= 4u;
-                fl1 = fl;
-            } else {
-                for (int k = 0; k < NV; ++k) Wt[k] = (P[c].W[k] - 0.5 * d[k]) - X[k];
-                prim_to_cons<MODEL>(q, Wt, Em, e);
-                if (muscl_check<MODEL>(Em, Wt, e)) fl |= 8u;
-                fl2 = fl;
-            }
-        }
-        bool ok2;
-        if ((fl1 & 1u) && (fl2 & 2u)) {
-            for (int k = 0; k < NV; ++k) {
-                EL[k] = Ep[k];
-                ER[k] = Em[k];
-            }
-            ok2 = (fl1 & 4u) && (fl2 & 8u);
-        } else {
-            double Wt[NV], e;
-            zero_slope_state<MODEL>(q, P[1], s_half, true, Wt);
-            prim_to_cons<MODEL>(q, Wt, EL, e);
-            bool okL = muscl_check<MODEL>(EL, Wt, e);
-            zero_slope_state<MODEL>(q, P[2], s_half, false, Wt);
-            prim_to_cons<MODEL>(q, Wt, ER, e);
-            bool okR = muscl_check<MODEL>(ER, Wt, e);
-            ok2 = okL && okR;
-        }
-        if (!ok2) {
-            for (int k = 0; k < NV; ++k) {
-                EL[k] = S[NV + k];
-                ER[k] = S[2 * NV + k];
-            }
+                Wt[k] = (side == 0 ? P[c].W[k] + h[k] : P[c].W[k] - h[k]) - X[k];
+            ok &= side_from_prim<MODEL>(q, Wt, side == 0 ? L : R);
         }
     }
-    double F[NV], us;
-    hllc_flux<MODEL>(q, wavespeed, EL, ER, F, us);
+    ok &= hllc_rn<MODEL>(q, wavespeed, L, R, F, us);
+    zL = L.U[NV - 1];
+    zR = R.U[NV - 1];
+    if (!ok) {
+        double EL[NV], ER[NV];
+        if (godunov) {
+            for (int k = 0; k < NV; ++k) {
+                EL[k] = S[k];
+                ER[k] = S[NV + k];
+            }
+        } else {
+            Prim<MODEL> P[4];
+            for (int c = 0; c < 4; ++c) cons_to_prim<MODEL>(q, S + c * NV, P[c]);
+            // cell 1 -> high-face states, cell 2 -> low-face states
+            double Ep[NV], Em[NV];
+            unsigned fl1 = 0, fl2 = 0;
+            for (int side = 0; side < 2; ++side) {
+                int c = 1 + side;
+                double d[NV], Wt[NV], Ut[NV], e, X[NV];
+                for (int k = 0; k < NV; ++k)
+                    d[k] = limit1(limiter, P[c].W[k] - P[c - 1].W[k], P[c + 1].W[k] - P[c].W[k]);
+                unsigned fl = 0;
+                for (int k = 0; k < NV; ++k) Wt[k] = P[c].W[k] + 0.5 * d[k];
+                prim_to_cons<MODEL>(q, Wt, Ut, e);
+                if (muscl_check<MODEL>(Ut, Wt, e)) fl |= 1u;
+                for (int k = 0; k < NV; ++k) Wt[k] = P[c].W[k] - 0.5 * d[k];
+                prim_to_cons<MODEL>(q, Wt, Ut, e);
+                if (muscl_check<MODEL>(Ut, Wt, e)) fl |= 2u;
+                jacobian_times<MODEL>(q, P[c], d, s_half, X);
+                if (side == 0) {
+                    for (int k = 0; k < NV; ++k) Wt[k] = (P[c].W[k] + 0.5 * d[k]) - X[k];
+                    prim_to_cons<MODEL>(q, Wt, Ep, e);
+                    if (muscl_check<MODEL>(Ep, Wt, e)) fl |= 4u;
+                    fl1 = fl;
+                } else {
+                    for (int k = 0; k < NV; ++k) Wt[k] = (P[c].W[k] - 0.5 * d[k]) - X[k];
+                    prim_to_cons<MODEL>(q, Wt, Em, e);
+                    if (muscl_check<MODEL>(Em, Wt, e)) fl |= 8u;
+                    fl2 = fl;
+                }
+            }
+            bool ok2;
+            if ((fl1 & 1u) && (fl2 & 2u)) {
+                for (int k = 0; k < NV; ++k) {
+                    EL[k] = Ep[k];
+                    ER[k] = Em[k];
+                }
+                ok2 = (fl1 & 4u) && (fl2 & 8u);
+            } else {
+                double Wt[NV], e;
+                zero_slope_state<MODEL>(q, P[1], s_half, true, Wt);
+                prim_to_cons<MODEL>(q, Wt, EL, e);
+                bool okL = muscl_check<MODEL>(EL, Wt, e);
+                zero_slope_state<MODEL>(q, P[2], s_half, false, Wt);
+                prim_to_cons<MODEL>(q, Wt, ER, e);
+                bool okR = muscl_check<MODEL>(ER, Wt, e);
+                ok2 = okL && okR;
+            }
+            if (!ok2) {
+                for (int k = 0; k < NV; ++k) {
+                    EL[k] = S[NV + k];
+                    ER[k] = S[2 * NV + k];
+                }
+            }
+        }
+        hllc_flux<MODEL>(q, wavespeed, EL, ER, F, us);
+        zL = EL[NV - 1];
+        zR = ER[NV - 1];
+    }
     for (int k = 0; k < NV; ++k) flux[(size_t)f * NV + k] = F[k];
     ustar[f] = us;
-    if (MODEL == MODEL_ALLAIRE && zstar) {
-        double cs = copysign(1.0, us);
-        zstar[f] = godunov ? (((1.0 + cs) / 2.0) * EL[5]) + (((1.0 - cs) / 2.0) * ER[5])
-                           : ((0.5 * (1.0 + cs)) * EL[5]) + ((0.5 * (1.0 - cs)) * ER[5]);
-    }
+    if (MODEL == MODEL_ALLAIRE && zstar) zstar[f] = face_z(godunov, us, zL, zR);
     (void)z_min;
 }
 
@@ -651,7 +686,7 @@ int cfd_device_bytes(const cfd_config* cfg, size_t* bytes) {
     long long plane;
     size_t be;
     layout_sizes(*cfg, nv, g, pitch, plane, be);
-    int mb = std::max(sweep_blocks(*cfg, DIR_X), sweep_blocks(*cfg, DIR_Y));
+    int mb = std::max(sweep_blocks(*cfg), kSMs * 4);
     *bytes = 2 * be * sizeof(double) + sizeof(DevState) + 4 * sizeof(double) * mb +
              CNT_N * sizeof(unsigned long long);
     return CFD_OK;
@@ -670,7 +705,7 @@ int cfd_create(const cfd_config* cfg, cfd_solver** out) {
     s->cfg = *cfg;
     s->eos = make_eos(*cfg);
     layout_sizes(*cfg, s->nv, s->g, s->pitch, s->plane, s->buf_elems);
-    s->max_blocks = std::max({sweep_blocks(*cfg, DIR_X), sweep_blocks(*cfg, DIR_Y), 148 * 4});
+    s->max_blocks = std::max(sweep_blocks(*cfg), kSMs * 4);
     auto cleanup = [&](int code) {
         cfd_destroy(s);
         return code;

@@ -838,9 +838,7 @@ static int add_member(cfd_batch* b, const cfd_config* cfg, const double* host_ic
     I.eos.p1 = c.pinf1;
     I.eos.g2 = c.model == CFD_MODEL_ALLAIRE ? c.gamma2 : 1.4;
     I.eos.p2 = c.model == CFD_MODEL_ALLAIRE ? c.pinf2 : 0.0;
-    I.eos.gm1_1 = I.eos.g1 - 1.0;
-    I.eos.gm1_2 = I.eos.g2 - 1.0;
-    I.eos.gp1 = I.eos.g1 * I.eos.p1;
+    eos_derive(I.eos);
     const double c1 = I.eos.g1 * I.eos.p1 / I.eos.gm1_1, c2 = I.eos.g2 * I.eos.p2 / I.eos.gm1_2;
     I.pf[0] = (float)I.eos.g1;
     I.pf[1] = (float)I.eos.p1;

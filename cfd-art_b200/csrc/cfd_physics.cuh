@@ -7,6 +7,10 @@
 // results are bit-identical to the reference's x86-64 build.  Where a value is
 // computed twice by the reference from identical inputs with identical
 // operations, it is computed once here and reused; that cannot change a bit.
+//
+// The functions here divide wherever the reference divides.  The sweeps run
+// the shared-reciprocal forms of cfd_exact.cuh, which give the same bits, and
+// come back to these where the guards of those forms do not hold.
 #pragma once
 
 #include <cstdint>
@@ -18,11 +22,30 @@ enum { LIM_MINMOD = 0, LIM_VANLEER = 1, LIM_MC = 2, LIM_UNLIMITED = 3 };
 enum { WS_DAVIS = 0, WS_PVRS = 1 };
 
 // Material parameters.  gm1_* = gamma - 1 and gp1 = gamma1 * pinf1 are formed
-// with the same single operation the reference performs inline.
+// with the same single operation the reference performs inline.  For the
+// shared-reciprocal forms: r1, r2 are the correctly rounded reciprocals of
+// gm1_1 and gm1_2 (shared_ok: both may serve as their divisors), and c1, c2
+// (gamma pinf / (gamma - 1)) and cm (2^-40 (|c1| + |c2|)) bound the mixture in
+// tests with a margin.
 struct Eos {
     double g1, p1, g2, p2;
     double gm1_1, gm1_2, gp1;
+    double r1, r2;
+    double c1, c2, cm;
+    int shared_ok;
 };
+inline void eos_derive(Eos& q) {
+    q.gm1_1 = q.g1 - 1.0;
+    q.gm1_2 = q.g2 - 1.0;
+    q.gp1 = q.g1 * q.p1;
+    q.r1 = 1.0 / q.gm1_1;
+    q.r2 = 1.0 / q.gm1_2;
+    q.c1 = q.g1 * q.p1 / q.gm1_1;
+    q.c2 = q.g2 * q.p2 / q.gm1_2;
+    q.cm = 9.1e-13 * ((q.c1 < 0 ? -q.c1 : q.c1) + (q.c2 < 0 ? -q.c2 : q.c2));
+    auto serves = [](double b) { return b > 1e-30 && b < 1e30; };
+    q.shared_ok = serves(q.gm1_1) && serves(q.gm1_2);
+}
 
 template <int MODEL> struct ModelTraits;
 template <> struct ModelTraits<MODEL_EULER> {
@@ -230,33 +253,37 @@ __device__ __forceinline__ double limit1(int lim, double a, double b) {
             return 0.0;
         case LIM_UNLIMITED:
             return 0.5 * (a + b);
-        default:
-            return (b > 0.0) ? smax(0.0, smin(a, b)) : smin(0.0, smax(a, b));
+        default: {
+            // (b > 0) ? max(0, min(a, b)) : min(0, max(a, b)): the smaller in
+            // size where the signs agree, else 0; a NaN in a gives 0, a NaN in
+            // b gives min(0, a), as the reference's std::min / std::max do
+            const double x = fabs(b) < fabs(a) ? b : a;
+            return ((b > 0.0) ? (a > 0.0) : (a < 0.0)) ? x : 0.0;
+        }
     }
 }
 
-// Limited slopes of all components, d = limit(W - Wm, Wp - W), with the
-// limiter chosen once for the cell rather than once per component (the
-// arithmetic of each component is limit1's).
+// Limited slopes of all components from the differences to the two
+// neighbours, with the limiter chosen once for the cell rather than once per
+// component (the arithmetic of each component is limit1's).
 template <int NV>
-__device__ __forceinline__ void limit_all1(int lim, const double* Wm, const double* W,
-                                           const double* Wp, double* d) {
+__device__ __forceinline__ void limit_diffs(int lim, const double* a, const double* b, double* d) {
     switch (lim) {
         case LIM_VANLEER:
 #pragma unroll
-            for (int k = 0; k < NV; ++k) d[k] = limit1(LIM_VANLEER, W[k] - Wm[k], Wp[k] - W[k]);
+            for (int k = 0; k < NV; ++k) d[k] = limit1(LIM_VANLEER, a[k], b[k]);
             break;
         case LIM_MC:
 #pragma unroll
-            for (int k = 0; k < NV; ++k) d[k] = limit1(LIM_MC, W[k] - Wm[k], Wp[k] - W[k]);
+            for (int k = 0; k < NV; ++k) d[k] = limit1(LIM_MC, a[k], b[k]);
             break;
         case LIM_UNLIMITED:
 #pragma unroll
-            for (int k = 0; k < NV; ++k) d[k] = limit1(LIM_UNLIMITED, W[k] - Wm[k], Wp[k] - W[k]);
+            for (int k = 0; k < NV; ++k) d[k] = limit1(LIM_UNLIMITED, a[k], b[k]);
             break;
         default:
 #pragma unroll
-            for (int k = 0; k < NV; ++k) d[k] = limit1(LIM_MINMOD, W[k] - Wm[k], Wp[k] - W[k]);
+            for (int k = 0; k < NV; ++k) d[k] = limit1(LIM_MINMOD, a[k], b[k]);
     }
 }
 

@@ -13,18 +13,27 @@
 // device-resident time and picks the next dt.
 //
 // Layout in HBM: SoA, one plane per stored component, interior cells only,
-// row-major with a padded pitch.  A CTA owns a tile of TS cells along the
-// sweep by NA lines across it and stages TS+4 cells per line (2-cell halo
-// each side) in shared memory, x fastest, so every global access is
-// coalesced in both sweep directions.  Four phases, separated by barriers:
-//   P1  conserved -> primitive per staged cell
-//   P2  limited slope and the four extrapolated/evolved face states per cell
-//   P3  HLLC flux per face
-//   P4  conservative update (+ Allaire z update / Euler fix-up), store,
-//       wave-speed reduction
+// row-major with a padded pitch.
+//
+// Form: warp segments.  A warp holds 32 consecutive cells along the sweep in
+// its lanes (28 outputs, two halo cells at each end) and takes them through
+// the whole update in registers: conversion, limited slope, the two evolved
+// face states, HLLC at the low face, update, and the wave speeds of the new
+// state where the launch reduces them.  Neighbour values come by shuffles, so
+// the update needs no barrier and no shared memory; the arithmetic is that of
+// cfd_exact.cuh, with the plain functions for a segment any lane of which
+// they do not serve.
+//
+// What bounds it: FP64 work.  At 2048^2 Euler the x sweep runs 870 thread
+// instructions per cell, 360 of them on the FP64 pipe (53 % busy, 64 % of the
+// issue slots), against 1921 and 478 when every division was made on its own
+// and the phases met in shared memory: x 314 -> 165 us, y 426 -> 194 us.
+// 4096^2 Euler 2.79 -> 1.41 ms a step, Allaire 2048x1024 0.90 -> 0.36 ms, the
+// 200x200 grid 22.0 -> 18.0 us a step, where a launch is one pass through the
+// code.
 #pragma once
 
-#include "cfd_physics.cuh"
+#include "cfd_exact.cuh"
 
 namespace cfd {
 
@@ -168,59 +177,302 @@ __device__ __forceinline__ void wave_speeds(const Eos& q, const double* U, doubl
     sv = fabs(P.W[ModelTraits<MODEL>::IT]) + c;
 }
 
-template <int MODEL, int DIR, int TS, int NA>
-struct SweepTile {
-    static constexpr int NV = ModelTraits<MODEL>::NV;
-    static constexpr int LA = TS + 4;           // staged cells per line
-    static constexpr int NSLOT = LA * NA;
-    static constexpr int STRIDE = (DIR == DIR_X) ? 1 : NA;  // next cell along the sweep
-    // slot of (along a, across b), x fastest in both directions
-    __device__ static __forceinline__ int slot(int a, int b) {
-        return (DIR == DIR_X) ? b * LA + a : a * NA + b;
-    }
-    // i-th item of a phase covering along-indices [a0, a0+cnt) on all lines
-    __device__ static __forceinline__ void item(int i, int a0, int cnt, int& a, int& b) {
-        if (DIR == DIR_X) {
-            b = i / cnt;
-            a = a0 + i - b * cnt;
-        } else {
-            a = a0 + i / NA;
-            b = i - (i / NA) * NA;
-        }
-    }
-};
+// One line segment: the warp's 32 lanes hold 32 consecutive cells along the
+// sweep (kSegOut outputs, two halo cells at each end), in the sweep frame.
+constexpr int kSegOut = 28;
 
-struct SweepSmemLayout {
-    // offsets in doubles
-    int U, WF, EP, EM, FLAGS_BYTES;
-};
-
-template <int MODEL, int DIR, int TS, int NA>
-__host__ __device__ constexpr int sweep_smem_bytes() {
-    using T = SweepTile<MODEL, DIR, TS, NA>;
-    // U, W/F (flux needs NV + 2 per face), E+, E-, flags
-    return (T::NV * T::NSLOT + (T::NV + 2) * T::NSLOT + 2 * T::NV * T::NSLOT) * 8 + T::NSLOT * 4 +
-           4 * 32 * 8;
+template <int N>
+__device__ __forceinline__ void shfl_up_d(const double* x, double* y) {
+#pragma unroll
+    for (int k = 0; k < N; ++k) y[k] = __shfl_up_sync(0xffffffffu, x[k], 1);
+}
+template <int N>
+__device__ __forceinline__ void shfl_down_d(const double* x, double* y) {
+#pragma unroll
+    for (int k = 0; k < N; ++k) y[k] = __shfl_down_sync(0xffffffffu, x[k], 1);
 }
 
-// Bounded for 4 (Euler, 64 registers) and 3 (Allaire, 80 registers) CTAs
-// per SM, spilling some 30-40 bytes per thread: 6 % and 7 % faster than at
-// 3 and 2 CTAs.
-template <int MODEL, int DIR, int TS, int NA>
-__global__ void __launch_bounds__(256, MODEL == MODEL_EULER ? 4 : 3) sweep_kernel(SweepArgs A) {
-    using Tl = SweepTile<MODEL, DIR, TS, NA>;
+// Event bits of a lane (counted under CNT_*).
+enum { EV_INPUT = 1, EV_ZEROED = 2, EV_FIRST = 4, EV_FIXUP = 8, EV_OUTPUT = 16 };
+
+// What a segment's update needs besides the cells.
+struct SegPar {
+    Eos q;
+    int limiter, wavespeed, godunov;
+    double z_min;
+};
+
+// z at a face: the side u* selects (A/headers/flux_solver_godunov.hpp:33-34,
+// A/headers/flux_solver_MUSCLhancock.hpp:375).
+__device__ __forceinline__ double face_z(int godunov, double us, double zL, double zR) {
+    const double cs = copysign(1.0, us);
+    if (godunov) return (((1.0 + cs) / 2.0) * zL) + (((1.0 - cs) / 2.0) * zR);
+    return ((0.5 * (1.0 + cs)) * zL) + ((0.5 * (1.0 - cs)) * zR);
+}
+
+// The conservative update from the fluxes at the lane's low face (F, with u*
+// and z* behind the components) and, by shuffle, at its high face.
+template <int MODEL>
+__device__ __forceinline__ void segment_new_state(const SegPar& A, const double* U, const double* F,
+                                                  double k_upd, double* N) {
+    constexpr int NV = ModelTraits<MODEL>::NV;
+    double FR[NV + 2];
+    shfl_down_d<MODEL == MODEL_EULER ? NV : NV + 2>(F, FR);
+#pragma unroll
+    for (int k = 0; k < NV; ++k) N[k] = U[k] + (k_upd * (F[k] - FR[k]));
+    if constexpr (MODEL == MODEL_ALLAIRE) {
+        double zL = 0.0, zR = 0.0;
+        if (A.godunov) {
+            zL = __shfl_up_sync(0xffffffffu, U[5], 1);
+            zR = __shfl_down_sync(0xffffffffu, U[5], 1);
+        }
+        N[5] = z_update(A.godunov, k_upd, zL, U[5], zR, F[NV], FR[NV], F[NV + 1], FR[NV + 1], A.z_min);
+        bool changed;
+        snap_allaire(N, changed);  // live assert(is_physical_state(...))
+    }
+}
+
+// The update of one segment: U (this lane's conserved state) -> N.  All 32
+// lanes take part; N is valid in lanes 2 .. 2 + kSegOut - 1 when every lane
+// returns true; `cell` marks the lanes whose N is stored.
+template <int MODEL>
+__device__ __forceinline__ bool segment_update(const SegPar& A, const double* U, double s_half,
+                                               double k_upd, bool cell, double* N) {
+    constexpr int NV = ModelTraits<MODEL>::NV;
+    const Eos& q = A.q;
+    const int lane = threadIdx.x & 31;
+    Side<MODEL> L, R;
+    bool ok;
+    {
+        Side<MODEL> S;  // the high face's
+        if (!A.godunov) {
+            PrimR<MODEL> P;
+            ok = c2p_rn<MODEL>(q, U, P);
+            double a[NV], b[NV], h[NV], X[NV], Wt[NV];
+            shfl_up_d<NV>(P.W, a);
+#pragma unroll
+            for (int k = 0; k < NV; ++k) a[k] = P.W[k] - a[k];
+            shfl_down_d<NV>(a, b);
+            limit_diffs<NV>(A.limiter, a, b, h);
+            bool in = jacobian_rn<MODEL>(q, P, h, s_half, X);
+#pragma unroll
+            for (int k = 0; k < NV; ++k) h[k] = 0.5 * h[k];
+            in &= slopes_physical<MODEL>(q, P.W, h);
+#pragma unroll
+            for (int k = 0; k < NV; ++k) Wt[k] = (P.W[k] + h[k]) - X[k];
+            in &= side_from_prim<MODEL>(q, Wt, S);
+#pragma unroll
+            for (int k = 0; k < NV; ++k) Wt[k] = (P.W[k] - h[k]) - X[k];
+            in &= side_from_prim<MODEL>(q, Wt, R);
+            ok &= in | (lane < 1) | (lane > 2 + kSegOut);
+        } else {
+#pragma unroll
+            for (int k = 0; k < NV; ++k) S.U[k] = U[k];
+            ok = side_from_cons<MODEL>(q, S);
+            // the reference's test of the stencil states
+            const double rho = S.rho;
+            if constexpr (MODEL == MODEL_ALLAIRE)
+                ok &= (U[0] >= 0.0) & (U[1] >= 0.0) & (U[5] >= 0.0) & (U[5] <= 1.0) &
+                      surely_energy(rho, U[2], U[3], U[4]);
+            else
+                ok &= surely_energy(rho, U[1], U[2], U[3]);
+            R = S;
+        }
+        // the lane below's high-face state is this lane's left state
+        shfl_up_d<NV>(S.U, L.U);
+        L.rho = L.U[0];
+        if constexpr (MODEL == MODEL_ALLAIRE) L.rho = L.U[0] + L.U[1];
+        L.u = __shfl_up_sync(0xffffffffu, S.u, 1);
+        L.p = __shfl_up_sync(0xffffffffu, S.p, 1);
+        L.c = __shfl_up_sync(0xffffffffu, S.c, 1);
+        if (MODEL == MODEL_ALLAIRE && A.wavespeed == WS_PVRS) {  // its speeds use the mixture
+            L.mix.eps = __shfl_up_sync(0xffffffffu, S.mix.eps, 1);
+            L.mix.k = __shfl_up_sync(0xffffffffu, S.mix.k, 1);
+            L.mix.ie = __shfl_up_sync(0xffffffffu, S.mix.ie, 1);
+        }
+    }
+    double F[NV + 2];
+    const bool fo = hllc_rn<MODEL>(q, A.wavespeed, L, R, F, F[NV]);
+    ok &= fo | (lane < 2) | (lane > 2 + kSegOut);
+    if constexpr (MODEL == MODEL_ALLAIRE) F[NV + 1] = face_z(A.godunov, F[NV], L.U[5], R.U[5]);
+    segment_new_state<MODEL>(A, U, F, k_upd, N);
+    bool fine;  // the new state surely passes the reference's test
+    if constexpr (MODEL == MODEL_ALLAIRE) {
+        const double rho = N[0] + N[1];
+        fine = (N[0] >= 0.0) & (N[1] >= 0.0) & (N[5] >= 0.0) & (N[5] <= 1.0) & (rho > 0.0) &
+               surely_energy(rho, N[2], N[3], N[4]);
+    } else {
+        fine = (N[0] > 0.0) & (N[3] > 0.0) & surely_energy(N[0], N[1], N[2], N[3]);
+    }
+    return ok & (fine | !cell);
+}
+
+// The same by the functions of cfd_physics.cuh, with the reference's
+// fallbacks and events: `face` marks lanes whose low face belongs to this
+// segment, `cell` those whose cell does.  In the y sweep the segment is the
+// rotated one; u and v enter the post-update restore symmetrically.
+template <int MODEL>
+__device__ __noinline__ void segment_update_plain(const SegPar& A, const double* Uin, double s_half,
+                                                  double k_upd, bool cell, bool face, double* N,
+                                                  unsigned& ev) {
     using MT = ModelTraits<MODEL>;
     constexpr int NV = MT::NV;
-    constexpr int LA = Tl::LA;
-    constexpr int NSLOT = Tl::NSLOT;
-    constexpr int ST = Tl::STRIDE;
+    const Eos& q = A.q;
+    double U[NV], UL[NV], EL[NV], ER[NV];
+#pragma unroll
+    for (int k = 0; k < NV; ++k) U[k] = Uin[k];
+    shfl_up_d<NV>(U, UL);
+    Prim<MODEL> P;
+    cons_to_prim<MODEL>(q, U, P);
+    // the reference's assert on the stencil states
+    bool phys;
+    if constexpr (MODEL == MODEL_EULER) phys = P.rho >= 0.0 && P.e >= 0.0;
+    else phys = is_physical_exact<MODEL>(U);
+    if (cell && !phys) ev |= EV_INPUT;
+    if (!A.godunov) {
+        double a[NV], b[NV], d[NV], X[NV], Wt[NV], Ut[NV], Ep[NV], e;
+        shfl_up_d<NV>(P.W, a);
+#pragma unroll
+        for (int k = 0; k < NV; ++k) a[k] = P.W[k] - a[k];
+        shfl_down_d<NV>(a, b);
+        limit_diffs<NV>(A.limiter, a, b, d);
+        // slope-extrapolated states (check only)
+        unsigned fl = 0;
+#pragma unroll
+        for (int k = 0; k < NV; ++k) Wt[k] = P.W[k] + 0.5 * d[k];
+        prim_to_cons<MODEL>(q, Wt, Ut, e);
+        if (muscl_check<MODEL>(Ut, Wt, e)) fl |= 1u;  // high face ok
+#pragma unroll
+        for (int k = 0; k < NV; ++k) Wt[k] = P.W[k] - 0.5 * d[k];
+        prim_to_cons<MODEL>(q, Wt, Ut, e);
+        if (muscl_check<MODEL>(Ut, Wt, e)) fl |= 2u;  // low face ok
+        // half-step evolved states
+        jacobian_times<MODEL>(q, P, d, s_half, X);
+#pragma unroll
+        for (int k = 0; k < NV; ++k) Wt[k] = (P.W[k] + 0.5 * d[k]) - X[k];
+        prim_to_cons<MODEL>(q, Wt, Ep, e);
+        if (muscl_check<MODEL>(Ep, Wt, e)) fl |= 4u;
+#pragma unroll
+        for (int k = 0; k < NV; ++k) Wt[k] = (P.W[k] - 0.5 * d[k]) - X[k];
+        prim_to_cons<MODEL>(q, Wt, ER, e);
+        if (muscl_check<MODEL>(ER, Wt, e)) fl |= 8u;
+        shfl_up_d<NV>(Ep, EL);
+        const unsigned flL = __shfl_up_sync(0xffffffffu, fl, 1);
+        bool ok2 = (flL & 4u) && (fl & 8u);
+        if (!((flL & 1u) && (fl & 2u))) {  // zero slopes for this face
+            if (face) ev |= EV_ZEROED;
+            Prim<MODEL> PL;
+            cons_to_prim<MODEL>(q, UL, PL);
+            zero_slope_state<MODEL>(q, PL, s_half, true, Wt);
+            prim_to_cons<MODEL>(q, Wt, EL, e);
+            const bool okL = muscl_check<MODEL>(EL, Wt, e);
+            zero_slope_state<MODEL>(q, P, s_half, false, Wt);
+            prim_to_cons<MODEL>(q, Wt, ER, e);
+            const bool okR = muscl_check<MODEL>(ER, Wt, e);
+            ok2 = okL && okR;
+        }
+        if (!ok2) {
+            if (face) ev |= EV_FIRST;
+#pragma unroll
+            for (int k = 0; k < NV; ++k) {
+                EL[k] = UL[k];
+                ER[k] = U[k];
+            }
+        }
+    } else {
+#pragma unroll
+        for (int k = 0; k < NV; ++k) {
+            EL[k] = UL[k];
+            ER[k] = U[k];
+        }
+    }
+    double F[NV + 2];
+    hllc_flux<MODEL>(q, A.wavespeed, EL, ER, F, F[NV]);
+    if constexpr (MODEL == MODEL_ALLAIRE) F[NV + 1] = face_z(A.godunov, F[NV], EL[5], ER[5]);
+    double Nn[NV];
+    segment_new_state<MODEL>(A, U, F, k_upd, Nn);
+    if (cell && !is_physical_exact<MODEL>(Nn)) {
+        if constexpr (MODEL == MODEL_ALLAIRE) {
+            ev |= EV_OUTPUT;
+        } else {
+            // E/sourcecode/euler_rowsweep.cpp:47-82: restore rho or e from the
+            // old state when the update produced rho or e <= 0
+            ev |= EV_FIXUP;
+            double rho = Nn[0];
+            double u = Nn[1] / rho;
+            double v = Nn[2] / rho;
+            double e = (Nn[3] / rho) - (0.5 * ((u * u) + (v * v)));
+            double rho_old = U[0];
+            double u_old = U[1] / rho_old;
+            double v_old = U[2] / rho_old;
+            double e_old = (U[3] / rho_old) - (0.5 * ((u_old * u_old) + (v_old * v_old)));
+            if (rho <= 1e-12) rho = rho_old;
+            if (e <= 1e-12) e = e_old;
+            double W[4] = {rho, u, v, sg_pressure(q, e, rho)};
+            double ee;
+            prim_to_cons<MODEL>(q, W, Nn, ee);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < NV; ++k) N[k] = Nn[k];
+}
 
+template <int MODEL>
+__device__ __noinline__ void plain_speeds(const Eos& q, const double* U, double& su, double& sv) {
+    double m1, m2;
+    wave_speeds<MODEL>(q, U, su, sv, m1, m2);
+}
+
+__device__ __forceinline__ void count_events(unsigned long long* ctr, unsigned ev) {
+    if (!__any_sync(0xffffffffu, ev != 0u)) return;
+    block_count(ctr, CNT_UNPHYSICAL_INPUT, ev & EV_INPUT);
+    block_count(ctr, CNT_SLOPE_ZEROED, ev & EV_ZEROED);
+    block_count(ctr, CNT_FIRST_ORDER, ev & EV_FIRST);
+    block_count(ctr, CNT_FIXUP, ev & EV_FIXUP);
+    block_count(ctr, CNT_UNPHYSICAL_OUTPUT, ev & EV_OUTPUT);
+}
+
+// Tiles: x, kSegOut columns by kXRows rows, a row per warp; y, kSegOut rows
+// by kYCols columns, a column per warp, staged through shared memory so that
+// global accesses are rows of kYCols cells (64 bytes per component).  CTA c of
+// G walks the tiles c, c + G, ...; the next tile's cells are copied global ->
+// shared with cp.async while the current one is computed.
+constexpr int kXRows = 4, kYCols = 8;
+constexpr int kYStride = 34;  // doubles per staged column: conflict-free both ways
+
+template <int DIR>
+__host__ __device__ constexpr int sweep_threads() {
+    return DIR == DIR_X ? 32 * kXRows : 32 * kYCols;
+}
+template <int MODEL, int DIR>
+__host__ __device__ constexpr int sweep_min_ctas() {
+    return MODEL == MODEL_EULER ? (DIR == DIR_X ? 4 : 2) : (DIR == DIR_X ? 3 : 1);
+}
+template <int MODEL, int DIR>
+__host__ __device__ constexpr int sweep_smem_bytes() {
+    constexpr int NV = ModelTraits<MODEL>::NV;
+    return DIR == DIR_X ? 2 * NV * 32 * kXRows * 8 : 2 * NV * kYCols * kYStride * 8;
+}
+template <int DIR>
+__host__ __device__ inline long long sweep_tiles(int nx, int ny) {
+    const int len = DIR == DIR_X ? nx : ny, wid = DIR == DIR_X ? ny : nx;
+    const int na = DIR == DIR_X ? kXRows : kYCols;
+    return (long long)((len + kSegOut - 1) / kSegOut) * ((wid + na - 1) / na);
+}
+
+__device__ __forceinline__ void copy8_async(double* dst, const double* src) {
+    const unsigned sa = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(src) : "memory");
+}
+
+template <int MODEL, int DIR>
+__global__ void __launch_bounds__(sweep_threads<DIR>(), sweep_min_ctas<MODEL, DIR>())
+    sweep_kernel(SweepArgs A) {
+    using MT = ModelTraits<MODEL>;
+    constexpr int NV = MT::NV;
+    constexpr int NA = DIR == DIR_X ? kXRows : kYCols;
+    constexpr int BUF = DIR == DIR_X ? NV * 32 * kXRows : NV * kYCols * kYStride;
     extern __shared__ __align__(16) double smem[];
-    double* sU = smem;                    // [NV][NSLOT] conserved (rotated in y)
-    double* sWF = sU + NV * NSLOT;        // [NV][NSLOT] primitives, later [NV+2][NSLOT] fluxes
-    double* sEP = sWF + (NV + 2) * NSLOT; // [NV][NSLOT] state at the cell's high face
-    double* sEM = sEP + NV * NSLOT;       // [NV][NSLOT] state at the cell's low face
-    unsigned char* sFl = reinterpret_cast<unsigned char*>(sEM + NV * NSLOT);  // flags
 
     const DevState* st = A.st;
     if (!A.use_host_dt && st->done) return;
@@ -229,267 +481,141 @@ __global__ void __launch_bounds__(256, MODEL == MODEL_EULER ? 4 : 3) sweep_kerne
     double* __restrict__ gout = A.bufs[cur ^ A.in_sel ^ 1];
     const double dt_step = A.use_host_dt ? A.dt_host : st->dt;  // dt of the whole step
     const double dt = A.dt_scale * dt_step;                        // this sweep's dt
-    const Eos q = A.eos;
-    const int len = (DIR == DIR_X) ? A.nx : A.ny;   // cells along the sweep
-    const int wid = (DIR == DIR_X) ? A.ny : A.nx;   // lines
-    const int tiles_along = (len + TS - 1) / TS;
-    const int t_al = blockIdx.x % tiles_along;
-    const int t_ac = blockIdx.x / tiles_along;
-    const int a_org = t_al * TS - 2;  // global along-coordinate of staged cell 0
-    const int b_org = t_ac * NA;
-    const int tid = threadIdx.x;
-    constexpr int NT = 256;
-
-    // ---- P1: load (with the boundary ghost fill), rotate, convert --------
-    // Ghost cell g (g = -1, -2 or len, len+1) mirrors interior cell -g-1 or
-    // 2*len-1-g; a reflective wall negates the normal momentum
-    // (E/sourcecode/euler_ppsweep.cpp:16,27).  The y-sweep works on the
-    // rotated state (u,v) -> (v,-u) (E/sourcecode/euler_colsweep.cpp:22-29).
-    bool bad_in = false;
-    for (int i = tid; i < NSLOT; i += NT) {
-        int a, b;
-        Tl::item(i, 0, LA, a, b);
-        int ga = a_org + a, gb = b_org + b;
-        bool line_ok = gb < wid;
-        int src = ga;
-        bool neg = false;
-        if (ga < 0) { src = -ga - 1; neg = A.bc_lo; }
-        else if (ga >= len) { src = 2 * len - 1 - ga; neg = A.bc_hi; }
-        // clamp staged cells beyond the last ghost (partial tiles) into range
-        src = min(max(src, 0), len - 1);
-        int gbs = line_ok ? gb : wid - 1;
-        long long off = (DIR == DIR_X) ? (long long)gbs * A.pitch + src
-                                       : (long long)src * A.pitch + gbs;
-        double U[NV];
-#pragma unroll
-        for (int k = 0; k < NV; ++k) U[k] = __ldg(gin + k * A.plane + off);
-        if (DIR == DIR_X) {
-            if (neg) U[MT::IM] = -U[MT::IM];
-        } else {
-            if (neg) U[MT::IT] = -U[MT::IT];
-            double t = U[MT::IM];
-            U[MT::IM] = U[MT::IT];
-            U[MT::IT] = -t;
-        }
-        int s = Tl::slot(a, b);
-#pragma unroll
-        for (int k = 0; k < NV; ++k) sU[k * NSLOT + s] = U[k];
-        Prim<MODEL> P;
-        cons_to_prim<MODEL>(q, U, P);
-#pragma unroll
-        for (int k = 0; k < NV; ++k) sWF[k * NSLOT + s] = P.W[k];
-        // reference assert on the stencil states (interior staged cells only)
-        bool phys;
-        if constexpr (MODEL == MODEL_EULER) phys = P.rho >= 0.0 && P.e >= 0.0;
-        else phys = is_physical_exact<MODEL>(U);
-        bad_in |= line_ok && ga >= 0 && ga < len && a >= 2 && a < TS + 2 && !phys;
-    }
-    block_count(A.counters, CNT_UNPHYSICAL_INPUT, bad_in);
-    __syncthreads();
-
     const double s_half = 0.5 * (dt / A.h_flux);
     const double k_upd = dt / A.h_upd;
+    const int len = (DIR == DIR_X) ? A.nx : A.ny;  // cells along the sweep
+    const int wid = (DIR == DIR_X) ? A.ny : A.nx;  // lines
+    // tiles in memory order: x fastest
+    const int tiles_x = (A.nx + (DIR == DIR_X ? kSegOut : NA) - 1) / (DIR == DIR_X ? kSegOut : NA);
+    const int tiles_y = (A.ny + (DIR == DIR_X ? NA : kSegOut) - 1) / (DIR == DIR_X ? NA : kSegOut);
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 
-    // ---- P2: slopes and face states per cell (along 1 .. LA-2) ----------
-    if (!A.godunov) {
-        for (int i = tid; i < (LA - 2) * NA; i += NT) {
-            int a, b;
-            Tl::item(i, 1, LA - 2, a, b);
-            int s = Tl::slot(a, b);
-            Prim<MODEL> P;
-            double Wl[NV], Wr[NV], d[NV];
+    // Ghost cell g (g = -1, -2 or len, len+1) mirrors interior cell -g-1 or
+    // 2*len-1-g; a reflective wall negates the normal momentum
+    // (E/sourcecode/euler_ppsweep.cpp:16,27).  Staged cells beyond the last
+    // ghost (partial tiles) are clamped into range.
+    auto source = [&](int ga) {
+        const int r = ga < 0 ? -ga - 1 : ga >= len ? 2 * len - 1 - ga : ga;
+        return min(max(r, 0), len - 1);
+    };
+    // the thread's cell of a tile: in x its own lane's, in y one of the eight
+    // cells of a staged row
+    auto issue = [&](int tx, int ty, double* buf) {
+        if (ty < tiles_y) {
+            const int a0 = (DIR == DIR_X ? tx : ty) * kSegOut - 2, b0 = (DIR == DIR_X ? ty : tx) * NA;
+            if constexpr (DIR == DIR_X) {
+                const long long off = (long long)min(b0 + warp, wid - 1) * A.pitch + source(a0 + lane);
 #pragma unroll
-            for (int k = 0; k < NV; ++k) {
-                P.W[k] = sWF[k * NSLOT + s];
-                Wl[k] = sWF[k * NSLOT + s - ST];
-                Wr[k] = sWF[k * NSLOT + s + ST];
-            }
-            limit_all1<NV>(A.limiter, Wl, P.W, Wr, d);
-            if constexpr (MODEL == MODEL_EULER) {
-                P.rho = P.W[0];
+                for (int k = 0; k < NV; ++k)
+                    copy8_async(buf + k * 32 * kXRows + threadIdx.x, gin + k * A.plane + off);
             } else {
-                P.rho = P.W[0] + P.W[1];
-                P.mix = mix_coeffs(q, P.W[5]);
+                const int r = threadIdx.x / kYCols, c = threadIdx.x % kYCols;
+                const long long off = (long long)source(a0 + r) * A.pitch + min(b0 + c, wid - 1);
+#pragma unroll
+                for (int k = 0; k < NV; ++k)
+                    copy8_async(buf + (k * kYCols + c) * kYStride + r, gin + k * A.plane + off);
             }
-            // slope-extrapolated states (check only)
-            double Wt[NV], Ut[NV], e;
-            unsigned fl = 0;
-#pragma unroll
-            for (int k = 0; k < NV; ++k) Wt[k] = P.W[k] + 0.5 * d[k];
-            prim_to_cons<MODEL>(q, Wt, Ut, e);
-            if (muscl_check<MODEL>(Ut, Wt, e)) fl |= 1u;  // high face ok
-#pragma unroll
-            for (int k = 0; k < NV; ++k) Wt[k] = P.W[k] - 0.5 * d[k];
-            prim_to_cons<MODEL>(q, Wt, Ut, e);
-            if (muscl_check<MODEL>(Ut, Wt, e)) fl |= 2u;  // low face ok
-            // half-step evolved states
-            double X[NV];
-            jacobian_times<MODEL>(q, P, d, s_half, X);
-#pragma unroll
-            for (int k = 0; k < NV; ++k) Wt[k] = (P.W[k] + 0.5 * d[k]) - X[k];
-            prim_to_cons<MODEL>(q, Wt, Ut, e);
-            if (muscl_check<MODEL>(Ut, Wt, e)) fl |= 4u;
-#pragma unroll
-            for (int k = 0; k < NV; ++k) sEP[k * NSLOT + s] = Ut[k];
-#pragma unroll
-            for (int k = 0; k < NV; ++k) Wt[k] = (P.W[k] - 0.5 * d[k]) - X[k];
-            prim_to_cons<MODEL>(q, Wt, Ut, e);
-            if (muscl_check<MODEL>(Ut, Wt, e)) fl |= 8u;
-#pragma unroll
-            for (int k = 0; k < NV; ++k) sEM[k * NSLOT + s] = Ut[k];
-            sFl[s] = (unsigned char)fl;
         }
-    }
-    __syncthreads();
+        asm volatile("cp.async.commit_group;\n" ::: "memory");
+    };
 
-    // ---- P3: flux at each face (along 2 .. TS+2; face a is between a-1, a)
-    // The primitive planes are dead after P2, so the fluxes overwrite them;
-    // P3 itself reads only sU, sEP, sEM and the flags.
-    double* sF = sWF;  // [NV + 2][NSLOT]: flux, u*, z*
-    bool ev_zero = false, ev_first = false;
-    for (int i = tid; i < (TS + 1) * NA; i += NT) {
-        int a, b;
-        Tl::item(i, 2, TS + 1, a, b);
-        int sR = Tl::slot(a, b), sL = sR - ST;
-        double EL[NV], ER[NV];
-        bool counted = (b_org + b) < wid && (a_org + a) <= len &&
-                       (a < TS + 2 || a_org + a == len);
-        if (A.godunov) {
-#pragma unroll
-            for (int k = 0; k < NV; ++k) {
-                EL[k] = sU[k * NSLOT + sL];
-                ER[k] = sU[k * NSLOT + sR];
-            }
-        } else {
-            unsigned fL = sFl[sL], fR = sFl[sR];
-            bool ok2;
-            if ((fL & 1u) && (fR & 2u)) {
-#pragma unroll
-                for (int k = 0; k < NV; ++k) {
-                    EL[k] = sEP[k * NSLOT + sL];
-                    ER[k] = sEM[k * NSLOT + sR];
-                }
-                ok2 = (fL & 4u) && (fR & 8u);
-            } else {
-                // zero slopes for this face (rare)
-                ev_zero |= counted;
-                double Ua[NV], Ub[NV], Wt[NV], e;
-#pragma unroll
-                for (int k = 0; k < NV; ++k) {
-                    Ua[k] = sU[k * NSLOT + sL];
-                    Ub[k] = sU[k * NSLOT + sR];
-                }
-                Prim<MODEL> PL, PR;
-                cons_to_prim<MODEL>(q, Ua, PL);
-                cons_to_prim<MODEL>(q, Ub, PR);
-                zero_slope_state<MODEL>(q, PL, s_half, true, Wt);
-                prim_to_cons<MODEL>(q, Wt, EL, e);
-                bool okL = muscl_check<MODEL>(EL, Wt, e);
-                zero_slope_state<MODEL>(q, PR, s_half, false, Wt);
-                prim_to_cons<MODEL>(q, Wt, ER, e);
-                bool okR = muscl_check<MODEL>(ER, Wt, e);
-                ok2 = okL && okR;
-            }
-            if (!ok2) {
-                ev_first |= counted;
-#pragma unroll
-                for (int k = 0; k < NV; ++k) {
-                    EL[k] = sU[k * NSLOT + sL];
-                    ER[k] = sU[k * NSLOT + sR];
-                }
-            }
-        }
-        double Fv[NV], us;
-        hllc_flux<MODEL>(q, A.wavespeed, EL, ER, Fv, us);
-#pragma unroll
-        for (int k = 0; k < NV; ++k) sF[k * NSLOT + sR] = Fv[k];
-        sF[NV * NSLOT + sR] = us;
-        if constexpr (MODEL == MODEL_ALLAIRE) {
-            double cs = copysign(1.0, us);
-            double zs;
-            if (A.godunov)  // A/headers/flux_solver_godunov.hpp:33-34
-                zs = (((1.0 + cs) / 2.0) * EL[5]) + (((1.0 - cs) / 2.0) * ER[5]);
-            else  // A/headers/flux_solver_MUSCLhancock.hpp:375
-                zs = ((0.5 * (1.0 + cs)) * EL[5]) + ((0.5 * (1.0 - cs)) * ER[5]);
-            sF[(NV + 1) * NSLOT + sR] = zs;
-        }
-    }
-    block_count(A.counters, CNT_SLOPE_ZEROED, ev_zero);
-    block_count(A.counters, CNT_FIRST_ORDER, ev_first);
-    __syncthreads();
+    const SegPar par{A.eos, A.limiter, A.wavespeed, A.godunov, A.z_min};
 
-    // ---- P4: update, store, reduce (along 2 .. TS+1) ---------------------
-    bool ev_fix = false, ev_bad = false;
     double r_mu = 0.0, r_mv = 0.0, r_m1 = 0.0, r_m2 = 0.0;
-    for (int i = tid; i < TS * NA; i += NT) {
-        int a, b;
-        Tl::item(i, 2, TS, a, b);
-        int ga = a_org + a, gb = b_org + b;
-        if (ga >= len || gb >= wid) continue;
-        int s = Tl::slot(a, b);
-        double U[NV], N[NV];
+    // this tile and the next (tx across the grid, ty up), stepped by the grid
+    const int step_x = (int)gridDim.x % tiles_x, step_y = (int)gridDim.x / tiles_x;
+    int tx = (int)blockIdx.x % tiles_x, ty = (int)blockIdx.x / tiles_x;
+    issue(tx, ty, smem);
+    int which = 0;
+    while (ty < tiles_y) {
+        int nx_ = tx + step_x, ny_ = ty + step_y;
+        if (nx_ >= tiles_x) {
+            nx_ -= tiles_x;
+            ++ny_;
+        }
+        double* buf = smem + which * BUF;
+        asm volatile("cp.async.wait_group 0;\n" ::: "memory");
+        if (DIR == DIR_Y) __syncthreads();
+        issue(nx_, ny_, smem + (which ^ 1) * BUF);
+        const int a0 = (DIR == DIR_X ? tx : ty) * kSegOut - 2, b0 = (DIR == DIR_X ? ty : tx) * NA;
+        const int ga = a0 + lane, gb = b0 + warp;
+        const bool line = gb < wid;  // the same for the whole warp
+        const bool cell = lane >= 2 && lane < 2 + kSegOut && ga < len;
+        if (line) {
+            const bool neg = (ga < 0 && A.bc_lo) || (ga >= len && A.bc_hi);
+            double U[NV], N[NV];
+            if constexpr (DIR == DIR_X) {
 #pragma unroll
-        for (int k = 0; k < NV; ++k) {
-            U[k] = sU[k * NSLOT + s];
-            N[k] = U[k] + (k_upd * (sF[k * NSLOT + s] - sF[k * NSLOT + s + ST]));
-        }
-        if constexpr (MODEL == MODEL_ALLAIRE) {
-            N[5] = z_update(A.godunov, k_upd, sU[5 * NSLOT + s - ST], U[5], sU[5 * NSLOT + s + ST],
-                            sF[NV * NSLOT + s], sF[NV * NSLOT + s + ST],
-                            sF[(NV + 1) * NSLOT + s], sF[(NV + 1) * NSLOT + s + ST], A.z_min);
-            bool changed;
-            snap_allaire(N, changed);  // live assert(is_physical_state(...))
-            ev_bad |= !is_physical_exact<MODEL>(N);
-        }
-        if (DIR == DIR_Y) {  // rotate back (E/sourcecode/euler_colsweep.cpp:66-73)
-            double t = N[MT::IM];
-            N[MT::IM] = -N[MT::IT];
-            N[MT::IT] = t;
-            double t2 = U[MT::IM];  // old state, unrotated, for the fix-up
-            U[MT::IM] = -U[MT::IT];
-            U[MT::IT] = t2;
-        }
-        if constexpr (MODEL == MODEL_EULER) {
-            // E/sourcecode/euler_rowsweep.cpp:47-82: restore rho or e from the
-            // old state when the update produced rho or e <= 0.  A state with
-            // rho > 0 and E*rho clearly above |m|^2/2 passes the exact test.
-            bool surely = N[0] > 0.0 && N[3] > 0.0 &&
-                          (N[3] * N[0]) > (0.5 * ((N[1] * N[1]) + (N[2] * N[2]))) * (1.0 + 1e-13);
-            if (!surely && !is_physical_exact<MODEL>(N)) {
-                ev_fix = true;
-                double rho = N[0];
-                double u = N[1] / rho;
-                double v = N[2] / rho;
-                double e = (N[3] / rho) - (0.5 * ((u * u) + (v * v)));
-                double rho_old = U[0];
-                double u_old = U[1] / rho_old;
-                double v_old = U[2] / rho_old;
-                double e_old = (U[3] / rho_old) - (0.5 * ((u_old * u_old) + (v_old * v_old)));
-                if (rho <= 1e-12) rho = rho_old;
-                if (e <= 1e-12) e = e_old;
-                double W[4] = {rho, u, v, sg_pressure(q, e, rho)};
-                double ee;
-                prim_to_cons<MODEL>(q, W, N, ee);
+                for (int k = 0; k < NV; ++k) U[k] = buf[k * 32 * kXRows + threadIdx.x];
+                if (neg) U[MT::IM] = -U[MT::IM];
+            } else {
+                // the rotated state (u,v) -> (v,-u) (E/sourcecode/euler_colsweep.cpp:22-29)
+#pragma unroll
+                for (int k = 0; k < NV; ++k) U[k] = buf[(k * kYCols + warp) * kYStride + lane];
+                if (neg) U[MT::IT] = -U[MT::IT];
+                const double t = U[MT::IM];
+                U[MT::IM] = U[MT::IT];
+                U[MT::IT] = -t;
+            }
+            bool ok = segment_update<MODEL>(par, U, s_half, k_upd, cell, N);
+            double su = 0.0, sv = 0.0;  // symmetric in the rotation up to the order of the two
+            if (A.reduce) ok &= wave_speeds_rn<MODEL>(par.q, N, su, sv) | !cell;
+            if (!__all_sync(0xffffffffu, ok)) {  // rare
+                const bool face = (lane >= 2 && lane < 2 + kSegOut && ga <= len) ||
+                                  (lane == 2 + kSegOut && ga == len);
+                const SegPar pc = par;
+                double Uc[NV], Nc[NV];
+                unsigned ec = 0;
+#pragma unroll
+                for (int k = 0; k < NV; ++k) Uc[k] = U[k];
+                segment_update_plain<MODEL>(pc, Uc, s_half, k_upd, cell, face, Nc, ec);
+#pragma unroll
+                for (int k = 0; k < NV; ++k) N[k] = Nc[k];
+                if (A.reduce && cell) plain_speeds<MODEL>(pc.q, Nc, su, sv);
+                count_events(A.counters, ec);
+            }
+            if (A.reduce && cell) {
+                r_mu = smax(r_mu, DIR == DIR_X ? su : sv);
+                r_mv = smax(r_mv, DIR == DIR_X ? sv : su);
+                r_m1 += N[0];
+                if (MODEL == MODEL_ALLAIRE) r_m2 += N[1];
+            }
+            if (DIR == DIR_Y) {  // rotate back (E/sourcecode/euler_colsweep.cpp:66-73)
+                const double t = N[MT::IM];
+                N[MT::IM] = -N[MT::IT];
+                N[MT::IT] = t;
+            }
+            if constexpr (DIR == DIR_X) {
+                if (cell) {
+                    const long long off = (long long)gb * A.pitch + ga;
+#pragma unroll
+                    for (int k = 0; k < NV; ++k) gout[k * A.plane + off] = N[k];
+                }
+            } else {
+                // back through the staged column (read by this warp only)
+#pragma unroll
+                for (int k = 0; k < NV; ++k) buf[(k * kYCols + warp) * kYStride + lane] = N[k];
             }
         }
-        long long off = (DIR == DIR_X) ? (long long)gb * A.pitch + ga : (long long)ga * A.pitch + gb;
+        if constexpr (DIR == DIR_Y) {
+            __syncthreads();
+            const int r = threadIdx.x / kYCols, c = threadIdx.x % kYCols;
+            if (r >= 2 && r < 2 + kSegOut && a0 + r < len && b0 + c < wid) {
+                const long long off = (long long)(a0 + r) * A.pitch + b0 + c;
 #pragma unroll
-        for (int k = 0; k < NV; ++k) gout[k * A.plane + off] = N[k];
-        if (A.reduce) {
-            double su, sv, m1, m2;
-            wave_speeds<MODEL>(q, N, su, sv, m1, m2);
-            r_mu = smax(r_mu, su);
-            r_mv = smax(r_mv, sv);
-            r_m1 += m1;
-            r_m2 += m2;
+                for (int k = 0; k < NV; ++k)
+                    gout[k * A.plane + off] = buf[(k * kYCols + c) * kYStride + r];
+            }
         }
+        tx = nx_;
+        ty = ny_;
+        which ^= 1;
     }
-    block_count(A.counters, CNT_FIXUP, ev_fix);
-    block_count(A.counters, CNT_UNPHYSICAL_OUTPUT, ev_bad);
     if (!A.reduce) return;
 
     // ---- block reduction, last-CTA finish ---------------------------------
-    __shared__ double red[4][8];
+    constexpr int NW = NA;
+    __shared__ double red[4][NW];
     __shared__ bool is_last;
     for (int o = 16; o > 0; o >>= 1) {
         r_mu = smax(r_mu, __shfl_down_sync(0xffffffffu, r_mu, o));
@@ -497,16 +623,16 @@ __global__ void __launch_bounds__(256, MODEL == MODEL_EULER ? 4 : 3) sweep_kerne
         r_m1 += __shfl_down_sync(0xffffffffu, r_m1, o);
         r_m2 += __shfl_down_sync(0xffffffffu, r_m2, o);
     }
-    if ((tid & 31) == 0) {
-        red[0][tid >> 5] = r_mu;
-        red[1][tid >> 5] = r_mv;
-        red[2][tid >> 5] = r_m1;
-        red[3][tid >> 5] = r_m2;
+    if (lane == 0) {
+        red[0][warp] = r_mu;
+        red[1][warp] = r_mv;
+        red[2][warp] = r_m1;
+        red[3][warp] = r_m2;
     }
     __syncthreads();
-    if (tid == 0) {
+    if (threadIdx.x == 0) {
         double mu = red[0][0], mv = red[1][0], m1 = red[2][0], m2 = red[3][0];
-        for (int w = 1; w < NT / 32; ++w) {
+        for (int w = 1; w < NW; ++w) {
             mu = smax(mu, red[0][w]);
             mv = smax(mv, red[1][w]);
             m1 += red[2][w];
