@@ -91,47 +91,49 @@ int launch_t(const MixedArgs& a, int sms, cudaStream_t st) {
     return CFD_OK;
 }
 
-// Resident 4-warp CTAs per SM of the marching sweep.
-template <int MODEL, int DIR>
-int march_per_sm() {
-    static int per_sm = 0;
-    if (!per_sm) {
-        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &per_sm, mixed_march_kernel<MODEL, DIR>, 128, march_smem_bytes<MODEL>());
-        if (e != cudaSuccess || per_sm < 1) per_sm = 1;
-    }
-    return per_sm;
+// The warp sweeps of the mixed form (4-warp CTAs): marching y sweep, segment
+// x sweep, each for one set of options.
+struct WarpKernel {
+    void (*fn)(MixedArgs);
+    int smem;
+};
+template <int MODEL, int OPT>
+WarpKernel warp_kernel(int dir) {
+    return dir == DIR_X ? WarpKernel{mixed_segment_x_kernel<MODEL, OPT>, seg_smem_bytes<MODEL>()}
+                        : WarpKernel{mixed_march_kernel<MODEL, OPT>, march_smem_bytes<MODEL>()};
 }
-
-// Persistent marching y sweep (4-warp CTAs): as many warps as fit on the
-// device (never more than there are strips), each walking every W-th strip.
-template <int MODEL, int DIR>
-int launch_march(const MixedArgs& a, int sms, cudaStream_t st) {
-    const int warps = std::max(1, std::min(a.ntiles, march_per_sm<MODEL, DIR>() * sms * 4));
-    mixed_march_kernel<MODEL, DIR><<<(warps + 3) / 4, 128, march_smem_bytes<MODEL>(), st>>>(a);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return cfd_fail(CFD_ERR_CUDA, "march launch: %s", cudaGetErrorString(e));
-    return CFD_OK;
-}
-
-// Persistent warp-segment x sweep (4-warp CTAs), launched like the marching one.
 template <int MODEL>
-int segment_per_sm() {
-    static int per_sm = 0;
-    if (!per_sm) {
-        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &per_sm, mixed_segment_x_kernel<MODEL>, 128, seg_smem_bytes<MODEL>());
-        if (e != cudaSuccess || per_sm < 1) per_sm = 1;
-    }
-    return per_sm;
+WarpKernel warp_kernel(int dir, int opt) {
+    if (opt == common_options<MODEL>(0)) return warp_kernel<MODEL, common_options<MODEL>(0)>(dir);
+    if (opt == common_options<MODEL>(1)) return warp_kernel<MODEL, common_options<MODEL>(1)>(dir);
+    return warp_kernel<MODEL, kOptGeneral>(dir);
+}
+WarpKernel warp_kernel(int model, int dir, int opt) {
+    return model == CFD_MODEL_EULER ? warp_kernel<MODEL_EULER>(dir, opt)
+                                    : warp_kernel<MODEL_ALLAIRE>(dir, opt);
 }
 
-template <int MODEL>
-int launch_segment(const MixedArgs& a, int sms, cudaStream_t st) {
-    const int warps = std::max(1, std::min(a.ntiles, segment_per_sm<MODEL>() * sms * 4));
-    mixed_segment_x_kernel<MODEL><<<(warps + 3) / 4, 128, seg_smem_bytes<MODEL>(), st>>>(a);
+// Resident CTAs per SM of such a kernel.
+int warp_per_sm(int model, int dir, int opt) {
+    static int known[2][2][MF_OPTIONS + 2] = {};
+    int& n = known[model][dir][opt + 1];
+    if (!n) {
+        const WarpKernel k = warp_kernel(model, dir, opt);
+        int v = 0;
+        const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k.fn, 128, k.smem);
+        n = e != cudaSuccess || v < 1 ? 1 : v;
+    }
+    return n;
+}
+
+// Persistent launch: as many warps as fit on the device (never more than
+// there are tiles), each walking every W-th tile.
+int launch_warp(int model, int dir, int opt, const MixedArgs& a, int sms, cudaStream_t st) {
+    const WarpKernel k = warp_kernel(model, dir, opt);
+    const int warps = std::max(1, std::min(a.ntiles, warp_per_sm(model, dir, opt) * sms * 4));
+    k.fn<<<(warps + 3) / 4, 128, k.smem, st>>>(a);
     cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return cfd_fail(CFD_ERR_CUDA, "segment launch: %s", cudaGetErrorString(e));
+    if (e != cudaSuccess) return cfd_fail(CFD_ERR_CUDA, "mixed sweep launch: %s", cudaGetErrorString(e));
     return CFD_OK;
 }
 
@@ -173,12 +175,11 @@ int launch_fast(int dir, const MixedArgs& a, int sms, cudaStream_t st) {
 }
 
 template <int MODEL>
-int launch_shape(int dir, int shape, const MixedArgs& a, int grid, cudaStream_t st) {
-    if (dir == DIR_X) return launch_segment<MODEL>(a, grid, st);
+int launch_shape(int dir, int shape, int opt, const MixedArgs& a, int grid, cudaStream_t st) {
+    if (dir == DIR_X || shape == kMarchShape) return launch_warp(MODEL, dir, opt, a, grid, st);
     switch (shape) {
         case 0: return launch_t<MODEL, DIR_Y, 28, 8>(a, grid, st);
         case 1: return launch_t<MODEL, DIR_Y, 60, 4>(a, grid, st);
-        case kMarchShape: return launch_march<MODEL, DIR_Y>(a, grid, st);
         default: return launch_t<MODEL, DIR_Y, 12, 16>(a, grid, st);
     }
 }
@@ -473,6 +474,7 @@ struct cfd_batch {
     struct Group {
         int model, fp64, dir, shape, ntiles, offset;
         int rows;  // marching strips: cells along the sweep per strip
+        int opt;   // the options all its members share, or kOptGeneral
     };
     std::vector<Group> groups;
     bool dirty = true;
@@ -527,6 +529,7 @@ int build_tables(cfd_batch* b) {
     // the strip length of a marching sweep; the fast FP64 form always
     // marches in y
     Shape shape_x[2][2], shape_y[2][2];
+    int opts[2][2];
     for (int model = 0; model < 2; ++model)
         for (int f64 = 0; f64 < 2; ++f64) {
             const int shp = f64 ? kMarchShape : b->shape[model][DIR_Y];
@@ -536,23 +539,26 @@ int build_tables(cfd_batch* b) {
             used = 0;
             b->seg_used[model][f64] = 0;
             std::vector<std::pair<int, int>> grids;
+            int& opt = opts[model][f64];
+            opt = kOptGeneral;
             for (const Member& m : b->members)
-                if (m.cfg.model == model && m.inst.fp64 == f64 && !m.final)
+                if (m.cfg.model == model && m.inst.fp64 == f64 && !m.final) {
+                    const int o = m.inst.flags & MF_OPTIONS;
+                    opt = grids.empty() || o == opt ? o : kOptGeneral;
                     grids.emplace_back(m.cfg.nx, m.cfg.ny);
+                }
             if (grids.empty()) continue;
             const int seg_sm =
                 f64 ? (model == CFD_MODEL_EULER ? segment64_per_sm<MODEL_EULER>()
                                                 : segment64_per_sm<MODEL_ALLAIRE>())
-                    : (model == CFD_MODEL_EULER ? segment_per_sm<MODEL_EULER>()
-                                                : segment_per_sm<MODEL_ALLAIRE>());
+                    : warp_per_sm(model, DIR_X, opt);
             shape_x[model][f64].na = seg_rows(grids, (long long)seg_sm * b->sms * 4);
             b->seg_used[model][f64] = shape_x[model][f64].na;
             if (shp != kMarchShape) continue;
             const int per_sm =
                 f64 ? (model == CFD_MODEL_EULER ? march64_per_sm<MODEL_EULER>()
                                                 : march64_per_sm<MODEL_ALLAIRE>())
-                    : (model == CFD_MODEL_EULER ? march_per_sm<MODEL_EULER, DIR_Y>()
-                                                : march_per_sm<MODEL_ALLAIRE, DIR_Y>());
+                    : warp_per_sm(model, DIR_Y, opt);
             shape_y[model][f64].ts = b->march_fixed[model]
                                          ? b->march_fixed[model]
                                          : march_rows(grids, (long long)per_sm * b->sms * 4);
@@ -584,6 +590,7 @@ int build_tables(cfd_batch* b) {
                 g.dir = dir;
                 g.shape = f64 ? (dir == DIR_X ? 0 : kMarchShape) : b->shape[model][dir];
                 g.offset = (int)all.size();
+                g.opt = opts[model][f64];
                 const Shape sh = dir == DIR_X ? shape_x[model][f64] : shape_y[model][f64];
                 g.rows = dir == DIR_X ? sh.na : sh.ts;
                 for (int idx : order) {
@@ -667,8 +674,8 @@ int enqueue_tick(cfd_batch* b, std::vector<Timed>* timing) {
                                                : launch_fast<MODEL_ALLAIRE>(dir, a, grid, b->stream);
             else
                 r = g.model == CFD_MODEL_EULER
-                        ? launch_shape<MODEL_EULER>(dir, g.shape, a, grid, b->stream)
-                        : launch_shape<MODEL_ALLAIRE>(dir, g.shape, a, grid, b->stream);
+                        ? launch_shape<MODEL_EULER>(dir, g.shape, g.opt, a, grid, b->stream)
+                        : launch_shape<MODEL_ALLAIRE>(dir, g.shape, g.opt, a, grid, b->stream);
             if (timing) {
                 cudaEventRecord(e1, b->stream);
                 timing->push_back({gi, e0, e1});
@@ -848,6 +855,11 @@ static int add_member(cfd_batch* b, const cfd_config* cfg, const double* host_ic
     I.pf[5] = (float)(1.0 / I.eos.gm1_2);
     I.pf[6] = (float)c1;
     I.pf[7] = (float)c2;
+    for (int k = 0; k < 2; ++k) {
+        const double z = k == 0 ? c.z_min : 1.0 - c.z_min;
+        I.zf[2 * k] = (float)z;
+        I.zf[2 * k + 1] = (float)(z - (double)I.zf[2 * k]);
+    }
     I.pd[0] = 1.0 / I.eos.gm1_1;
     I.pd[1] = 1.0 / I.eos.gm1_2;
     I.pd[2] = c1;

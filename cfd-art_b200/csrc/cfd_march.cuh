@@ -10,14 +10,18 @@
 // starts from it.  The strip length is chosen per launch on the
 // host (kMarchMinRows..kMarchMaxRows) so that the strips fill the resident
 // warps.  No barrier is needed, and only the two halo cells at each end of
-// a strip are re-read.  In the y sweep the lanes are 32 consecutive columns,
-// so every step reads 32 consecutive cells (coalesced).  The code also has
-// the x form (lanes on 32 rows, each lane reading consecutive cells of its
-// row step by step), but on B200 that form measured 1.9x slower than the
-// tiled x sweep, so the batch marches in y only.  The arithmetic of every
+// a strip are re-read.  The lanes are 32 consecutive columns, so every step
+// reads 32 consecutive cells (coalesced).  (Marching along x, with the lanes
+// on 32 rows, measured 1.9x slower than the tiled x sweep.)  The arithmetic of every
 // cell, face and update is the one of the tiled sweep (cfd_mixed.cuh): the
 // same functions in the same order, so the two give the same results bit for
 // bit and the autotuner may pick either.
+//
+// Both sweeps are compiled for the common options (limiter, PVRS speeds,
+// stiffened gas) as well: a member's options come from memory, so the compiler
+// cannot see that a branch on them is uniform and pays for reconvergence at
+// every one.  A launch all of whose members have one such set of options runs
+// its instantiation, any other the general one.
 //
 // Reduction: each strip reduces its lanes' wave speeds and masses into its
 // own slot of the instance's partials; the strip that completes the
@@ -35,6 +39,10 @@ namespace mixed {
 
 constexpr int kMarchMaxRows = 64, kMarchMinRows = 16;  // rows of a strip (its width is one warp)
 
+template <bool B> struct Bool {
+    static constexpr bool value = B;
+};
+
 // y-sweep frame: the boundary sign of a mirrored row, then (u, v) -> (v, -u).
 template <int MODEL>
 __device__ __forceinline__ void march_rotate_in(float* h, float* l, bool neg) {
@@ -48,19 +56,6 @@ __device__ __forceinline__ void march_rotate_in(float* h, float* l, bool neg) {
     l[MT::IM] = l[MT::IT];
     h[MT::IT] = -t;
     l[MT::IT] = -tl;
-}
-
-// Sweep frame of a loaded cell: the boundary sign of a mirrored cell (normal
-// momentum), and in y the rotation (u, v) -> (v, -u).
-template <int MODEL, int DIR>
-__device__ __forceinline__ void march_frame_in(float* h, float* l, bool neg) {
-    using MT = ModelTraits<MODEL>;
-    if (DIR == DIR_Y) {
-        march_rotate_in<MODEL>(h, l, neg);
-    } else if (neg) {
-        h[MT::IM] = -h[MT::IM];
-        l[MT::IM] = -l[MT::IM];
-    }
 }
 
 // Last-strip finish of the wave-speed reduction, by one warp: slots in slot
@@ -99,17 +94,17 @@ __device__ __forceinline__ void march_finish(DevState* st, const double* partial
 }
 
 // Rows staged through shared memory with cp.async (no registers held by the
-// loads in flight): a ring of kMSlots slots per lane holding rows k-2 .. k+3
-// while row k is computed; kMAhead rows in flight, row k + kMAhead issued
-// into the slot of row k - 3 once row k has arrived; per slot MU 16-byte
-// units per lane (value and compensation words of components 0-3; for
+// loads in flight): a ring of kMSlots slots per lane holding at least rows
+// k-2 .. k+3 while row k is computed; kMAhead rows in flight; per slot MU
+// 16-byte units per lane (value and compensation words of components 0-3; for
 // Allaire E and z with their compensation words).  The raw cells of row
 // k-2, which its update starts from, are therefore read again from the
-// ring rather than carried in registers for two rows: 124 -> 115 registers
-// for Euler and 5 % less time per y sweep; Allaire's carried window (face
-// state, flux) then fits in its 128 registers, where it had to sit in
-// shared memory before.
-constexpr int kMAhead = 3, kMSlots = kMAhead + 3;
+// ring rather than carried in registers for two rows.  Six slots would do; with
+// eight a slot's offset is a mask (4 instructions a row fewer).
+//
+// Element offsets within a plane are 32-bit: a plane has at most 2^31 cells
+// and its row padding, and an address is then one multiply-add.
+constexpr int kMAhead = 3, kMSlots = 8;
 template <int MODEL>
 __host__ __device__ constexpr int march_units() {
     return MODEL == MODEL_ALLAIRE ? 3 : 2;
@@ -122,58 +117,68 @@ __host__ __device__ constexpr int march_smem_bytes() {
 }
 
 // Starts copying the cell at element offset `off` of the planes `Q` (value
-// and compensation words) into slot `s` of this lane's staging ring `stg`.
+// and compensation words) into a slot of this lane's staging ring.
 template <int MODEL>
-__device__ __forceinline__ void mstage_issue(char* stg, int s, const MPlanes& Q, long long off) {
-    constexpr int MU = march_units<MODEL>();
-    cp_async16(stg + ((s * MU + 0) * 32) * 16, Q.v4 + off);
-    cp_async16(stg + ((s * MU + 1) * 32) * 16, Q.c4 + off);
+__device__ __forceinline__ void mstage_issue(char* slot, const MPlanes& Q, unsigned off) {
+    cp_async16(slot, Q.v4 + off);
+    cp_async16(slot + 512, Q.c4 + off);
     if constexpr (MODEL == MODEL_ALLAIRE) {
-        cp_async8(stg + ((s * MU + 2) * 32) * 16, Q.v2 + off);
-        cp_async8(stg + ((s * MU + 2) * 32) * 16 + 8, Q.c2 + off);
+        cp_async8(slot + 1024, Q.v2 + off);
+        cp_async8(slot + 1024 + 8, Q.c2 + off);
     }
 }
 
-// The cell staged in slot `s` (as stored: no mirror, no rotation).
+// The cell staged in a slot (as stored: no mirror, no rotation).
 template <int MODEL>
-__device__ __forceinline__ void mstage_read(const char* stg, int s, float* h, float* l) {
-    constexpr int MU = march_units<MODEL>();
-    const float4 a = *reinterpret_cast<const float4*>(stg + ((s * MU + 0) * 32) * 16);
-    const float4 b = *reinterpret_cast<const float4*>(stg + ((s * MU + 1) * 32) * 16);
+__device__ __forceinline__ void mstage_read(const char* slot, float* h, float* l) {
+    const float4 a = *reinterpret_cast<const float4*>(slot);
+    const float4 b = *reinterpret_cast<const float4*>(slot + 512);
     h[0] = a.x; h[1] = a.y; h[2] = a.z; h[3] = a.w;
     l[0] = b.x; l[1] = b.y; l[2] = b.z; l[3] = b.w;
     if constexpr (MODEL == MODEL_ALLAIRE) {
-        const float4 e = *reinterpret_cast<const float4*>(stg + ((s * MU + 2) * 32) * 16);
+        const float4 e = *reinterpret_cast<const float4*>(slot + 1024);
         h[4] = e.x; h[5] = e.y;
         l[4] = e.z; l[5] = e.w;
     }
 }
 
-// One strip: cells [r0, r1) along the sweep of lines [b_org, b_org + 32) of
-// instance g.inst ("row" below means a position along the sweep).
-template <int MODEL, int DIR>
+// The options of a member as the sweeps branch on them (Inst::flags without
+// the walls), and the sets of them that have their own instantiations: minmod
+// and van Leer slopes of a gas (Euler), minmod slopes with PVRS speeds of a
+// stiffened gas and minmod slopes of two gases (Allaire).
+constexpr int MF_OPTIONS = 31;
+constexpr int kOptGeneral = -1;
+template <int MODEL> __host__ __device__ constexpr int common_options(int i) {
+    return MODEL == MODEL_EULER ? (i == 0 ? LIM_MINMOD : LIM_VANLEER)
+                                : (i == 0 ? (LIM_MINMOD | MF_PVRS | MF_STIFF) : LIM_MINMOD);
+}
+
+// One strip: rows [r0, r1) of the columns [b_org, b_org + 32) of instance
+// g.inst.
+template <int MODEL, int OPT>
 __device__ __forceinline__ void march_strip(const MixedArgs& A, const TileGeom& g) {
     using MT = ModelTraits<MODEL>;
     constexpr int NV = MT::NV;
     const int lane = threadIdx.x & 31;
     const Inst& I = A.insts[g.inst];
-    const MPar P = load_par(I);
+    MPar P = load_par(I);
+    const bool wall_lo = (P.flags >> 7) & 1, wall_hi = (P.flags >> 8) & 1;  // bottom, top
+    if (OPT != kOptGeneral) P.flags = OPT;
     DevState* st = I.st;
     const double dt = st->dt;
-    const double h_flux = DIR == DIR_X ? I.dx : (I.fix_dy ? I.dy : I.dx);
-    const float s_half = (float)(0.5 * (dt / h_flux));
-    const float k_upd = (float)(dt / (DIR == DIR_X ? I.dx : I.dy));
-    const int ny = g.len, nx = g.wid;  // cells along the sweep, lines
-    const int col = g.b_org + lane;    // this lane's line
+    const float s_half = (float)(0.5 * (dt / (I.fix_dy ? I.dy : I.dx)));
+    const float k_upd = (float)(dt / I.dy);
+    const int ny = g.len, nx = g.wid;
+    const int col = g.b_org + lane;
     const bool live = col < nx;
     const int c = min(col, nx - 1);
     const int r0 = g.a_org + 2;
     const int r1 = min(r0 + A.rows, ny);
-    // the x sweep reads the current buffer, the y sweep the x sweep's output
-    const int bin = DIR == DIR_X ? g.cur : g.cur ^ 1, bout = bin ^ 1;
-    // Euler holds the planes in registers (2 % faster); Allaire, at its
-    // 128-register limit, spilled that way and measured 3 % slower, so it
-    // reads them from the member descriptor where it uses them
+    // the y sweep reads the x sweep's output.  Euler holds the planes in
+    // registers (2 % faster); Allaire, at its 128-register limit, spilled that
+    // way and measured 3 % slower, so it reads them from the member descriptor
+    // where it uses them
+    const int bin = g.cur ^ 1, bout = g.cur;
     const MPlanes qin_r = mplanes<MODEL>(I, bin), qout_r = mplanes<MODEL>(I, bout);
     auto qin = [&] {
         if constexpr (MODEL == MODEL_EULER) return qin_r;
@@ -183,9 +188,7 @@ __device__ __forceinline__ void march_strip(const MixedArgs& A, const TileGeom& 
         if constexpr (MODEL == MODEL_EULER) return qout_r;
         else return mplanes<MODEL>(I, bout);
     };
-    const long long pitch = I.pitch;
-    const int wall_bit = DIR == DIR_X ? 5 : 7;  // walls L, R / B, T
-    const bool wall_lo = (P.flags >> wall_bit) & 1, wall_hi = (P.flags >> (wall_bit + 1)) & 1;
+    const unsigned pitch = I.pitch;
     const bool god = P.godunov();
     const int lim = P.limiter();
 
@@ -204,7 +207,7 @@ __device__ __forceinline__ void march_strip(const MixedArgs& A, const TileGeom& 
     };
 
     float W1[NV], W2[NV];       // W(k-1), W(k-2)
-    unsigned flp = 0;           // physicality flags of row k-2
+    bool okp = false;           // whether Pp may be used
     float Pp[NV], Fl[NV];       // state at the high face of row k-2, flux at its low face
     float us_low = 0.f, zs_low = 0.f;
     float z3 = 0.f;             // z of row k-3 (first-order z update)
@@ -213,64 +216,60 @@ __device__ __forceinline__ void march_strip(const MixedArgs& A, const TileGeom& 
 #pragma unroll
     for (int q = 0; q < NV; ++q) W1[q] = W2[q] = Pp[q] = Fl[q] = 0.f;
 
-    // rows staged ahead (y sweep: line = column, along = row)
     extern __shared__ __align__(16) char march_stage[];
     constexpr int MU = march_units<MODEL>();
-    char* stg = march_stage + (threadIdx.x >> 5) * (kMSlots * MU * 32 * 16) +
-                16 * lane;
-    auto issue = [&](int s, int k) {
-        bool ng;
-        mstage_issue<MODEL>(stg, s, qin(), (long long)src_row(k, ng) * pitch + c);
-    };
-    auto staged = [&](int s, float* h, float* l) { mstage_read<MODEL>(stg, s, h, l); };
+    constexpr int SB = MU * 32 * 16, RB = kMSlots * SB;  // bytes of a slot, of the ring
+    char* stg = march_stage + (threadIdx.x >> 5) * RB + 16 * lane;
+    bool ng;
 #pragma unroll
     for (int j = 0; j < kMAhead; ++j) {
-        if (r0 - 2 + j <= r1 + 1) issue(j, r0 - 2 + j);
+        if (r0 - 2 + j <= r1 + 1)
+            mstage_issue<MODEL>(stg + j * SB, qin(), (unsigned)src_row(r0 - 2 + j, ng) * pitch + c);
         cp_async_commit();
     }
-    int slot = 0;
+    // the ring's slots are numbered by row: row r0 - 2 + j is in slot j mod
+    // kMSlots; `at` is row k's
+    int at = 0;
+    auto slot_of = [&](int rows) {  // of row k + rows
+        static_assert((kMSlots & (kMSlots - 1)) == 0, "a power of two");
+        return stg + (unsigned)((at + rows) & (kMSlots - 1)) * SB;
+    };
 
-    for (int k = r0 - 2; k <= r1 + 1; ++k) {
+    // Row k arrives.  `steady`: k - 2 >= r0 and k + kMAhead < r1, so every
+    // part of the step applies and no row in it is mirrored.
+    auto row_step = [&](int k, auto steady_t) {
+        constexpr bool steady = decltype(steady_t)::value;
         float h[NV], l[NV];
-        bool neg;
-        src_row(k, neg);
         asm volatile("cp.async.wait_group %0;\n" ::"n"(kMAhead - 1) : "memory");
-        staged(slot, h, l);
-        // row k + kMAhead into the slot of row k - 3 (read three rows ago)
-        if (k + kMAhead <= r1 + 1) issue(slot >= 3 ? slot - 3 : slot + kMSlots - 3, k + kMAhead);
+        mstage_read<MODEL>(slot_of(0), h, l);
+        bool neg = false;
+        if (steady) {
+            mstage_issue<MODEL>(slot_of(kMAhead), qin(), (unsigned)(k + kMAhead) * pitch + c);
+        } else {
+            if (k + kMAhead <= r1 + 1)
+                mstage_issue<MODEL>(slot_of(kMAhead), qin(),
+                                    (unsigned)src_row(k + kMAhead, neg) * pitch + c);
+            src_row(k, neg);
+        }
         cp_async_commit();
-        const int slot2 = slot >= 2 ? slot - 2 : slot + kMSlots - 2;  // row k - 2
-        slot = slot == kMSlots - 1 ? 0 : slot + 1;
-        march_frame_in<MODEL, DIR>(h, l, neg);
+        march_rotate_in<MODEL>(h, l, neg);
         float W0[NV];
         c2p_mixed<MODEL>(I, P, h, l, W0);
 
         // slopes and evolved face states of row k-1
         float Pn[NV], Mn[NV];
-        unsigned fln = 0;
-        if (k >= r0 && !god) {
-            float d[NV], X[NV];
+        bool okn = false, okm = false;
+        if ((steady || k >= r0) && !god) {
+            float d[NV];
             limit_all<NV>(lim, W2, W1, W0, d);
-#pragma unroll
-            for (int q = 0; q < NV; ++q) Pn[q] = W1[q] + 0.5f * d[q];
-            if (phys_prim<MODEL>(P, Pn)) fln |= 1u;
-#pragma unroll
-            for (int q = 0; q < NV; ++q) Pn[q] = W1[q] - 0.5f * d[q];
-            if (phys_prim<MODEL>(P, Pn)) fln |= 2u;
-            jac_f<MODEL>(P, W1, d, s_half, X);
-#pragma unroll
-            for (int q = 0; q < NV; ++q) Pn[q] = (W1[q] + 0.5f * d[q]) - X[q];
-            if (phys_prim<MODEL>(P, Pn)) fln |= 4u;
-#pragma unroll
-            for (int q = 0; q < NV; ++q) Mn[q] = (W1[q] - 0.5f * d[q]) - X[q];
-            if (phys_prim<MODEL>(P, Mn)) fln |= 8u;
+            face_states<MODEL>(P, W1, d, s_half, Pn, Mn, okn, okm);
         }
 
         // HLLC at the face between rows k-2 and k-1
         float Fh[NV + 2];
-        if (k >= r0 + 1) {
+        if (steady || k >= r0 + 1) {
             float WL[NV], WR[NV];
-            const bool second = !god && (flp & 1u) && (fln & 2u) && (flp & 4u) && (fln & 8u);
+            const bool second = okp && okm;  // else first order
 #pragma unroll
             for (int q = 0; q < NV; ++q) {
                 WL[q] = second ? Pp[q] : W2[q];
@@ -280,16 +279,12 @@ __device__ __forceinline__ void march_strip(const MixedArgs& A, const TileGeom& 
         }
 
         // compensated update of row k-2
-        if (k >= r0 + 2) {
-            const int row = k - 2;  // inside [r0, r1): no mirror, no sign
+        if (steady || k >= r0 + 2) {
+            const unsigned off = (unsigned)(k - 2) * pitch + c;  // inside [r0, r1): no mirror
             float hh[NV], ll[NV];
-            staged(slot2, hh, ll);  // row k-2 as loaded (inside: no mirror)
-            march_frame_in<MODEL, DIR>(hh, ll, false);
-#pragma unroll
-            for (int q = 0; q < NV; ++q) {
-                if (MODEL == MODEL_ALLAIRE && q == 5) continue;
-                comp_add(hh[q], ll[q], k_upd * (Fl[q] - Fh[q]));
-            }
+            mstage_read<MODEL>(slot_of(-2), hh, ll);
+            march_rotate_in<MODEL>(hh, ll, false);
+            comp_update<NV>(hh, ll, k_upd, Fl, Fh);
             if constexpr (MODEL == MODEL_ALLAIRE) {
                 const float usL = us_low, usR = Fh[NV], zsL = zs_low, zsR = Fh[NV + 1];
                 const float z = hh[5];
@@ -303,7 +298,7 @@ __device__ __forceinline__ void march_strip(const MixedArgs& A, const TileGeom& 
                 if (hh[0] < 0.0f) { hh[0] = 0.0f; ll[0] = 0.0f; }
                 if (hh[1] < 0.0f) { hh[1] = 0.0f; ll[1] = 0.0f; }
             }
-            if (DIR == DIR_Y) {  // rotate back
+            {  // rotate back
                 float t = hh[MT::IM], tl = ll[MT::IM];
                 hh[MT::IM] = -hh[MT::IT];
                 ll[MT::IM] = -ll[MT::IT];
@@ -316,8 +311,7 @@ __device__ __forceinline__ void march_strip(const MixedArgs& A, const TileGeom& 
                 // density / energy restore as in the plain form (rare)
                 if (!(hh[0] > 1e-12f) || !(Wn[3] + P.gp1 > 0.0f)) {
                     float oh[NV], ol[NV], Wo[NV];  // the cell before the update
-                    load_cell<MODEL>(qin(), DIR == DIR_Y ? (long long)row * pitch + c : (long long)c * pitch + row,
-                                     oh, ol);
+                    load_cell<MODEL>(qin(), off, oh, ol);
                     c2p_mixed<MODEL>(I, P, oh, ol, Wo);  // stored (unrotated) frame
                     float rho = hh[0] > 1e-12f ? hh[0] : oh[0];
                     float u = Wn[1], v = Wn[2];
@@ -331,12 +325,7 @@ __device__ __forceinline__ void march_strip(const MixedArgs& A, const TileGeom& 
                 }
             }
             if (live) {
-                store_cell<MODEL>(qout(),
-                                  DIR == DIR_Y ? (long long)row * pitch + c
-                                               : (long long)c * pitch + row,
-                                  hh, ll);
-            }
-            if (DIR == DIR_Y && live) {
+                store_cell<MODEL>(qout(), off, hh, ll);
                 float cs = sound_f<MODEL>(P, Wn);
                 rmu = fmaxf_s(rmu, fabsf(Wn[MT::IM]) + cs);
                 rmv = fmaxf_s(rmv, fabsf(Wn[MT::IT]) + cs);
@@ -353,16 +342,28 @@ __device__ __forceinline__ void march_strip(const MixedArgs& A, const TileGeom& 
             W1[q] = W0[q];
             Pp[q] = Pn[q];
         }
-        flp = fln;
-        if (k >= r0 + 1) {
+        okp = okn;
+        ++at;
+        if (steady || k >= r0 + 1) {
 #pragma unroll
             for (int q = 0; q < NV; ++q) Fl[q] = Fh[q];
             us_low = Fh[NV];
             zs_low = MODEL == MODEL_ALLAIRE ? Fh[NV + 1] : 0.f;
         }
+    };
+    int k = r0 - 2;
+    while (k <= r1 + 1) {
+        row_step(k, Bool<false>{});
+        ++k;
+        // Euler: the rows away from the strip's ends run a copy of the step
+        // without its tests, unrolled by two so that half the window changes
+        // roles instead of being copied (6 % faster in all); Allaire spills
+        // with the two copies (5 % slower)
+        if (MODEL == MODEL_EULER && k == r0 + 2)
+#pragma unroll 2
+            for (; k + kMAhead < r1; ++k) row_step(k, Bool<true>{});
     }
 
-    if (DIR == DIR_X) return;  // the y sweep reduces
     // this strip's wave speeds and masses into its slot, then the ticket
     double mu = (double)rmu, mv = (double)rmv;
     for (int o = 16; o > 0; o >>= 1) {
@@ -392,13 +393,13 @@ __device__ __forceinline__ void march_strip(const MixedArgs& A, const TileGeom& 
 // w + W, w + 2W, ... of the launch's strip list, so the strips of members
 // that have finished (skipped) are spread over all warps instead of idling
 // some of them.
-template <int MODEL, int DIR>
-__global__ void __launch_bounds__(128) mixed_march_kernel(MixedArgs A) {
+template <int MODEL, int OPT>
+__global__ void __launch_bounds__(128, 4) mixed_march_kernel(MixedArgs A) {
     const int gw = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int nw = gridDim.x * (blockDim.x >> 5);
     for (int tile = gw; tile < A.ntiles; tile += nw) {
-        const TileGeom g = tile_geom<DIR, kMarchMaxRows, 32>(A, tile);
-        if (!g.skip) march_strip<MODEL, DIR>(A, g);
+        const TileGeom g = tile_geom<DIR_Y, kMarchMaxRows, 32>(A, tile);
+        if (!g.skip) march_strip<MODEL, OPT>(A, g);
     }
 }
 
@@ -410,20 +411,13 @@ __global__ void __launch_bounds__(128) mixed_march_kernel(MixedArgs A) {
 // come from the adjacent lanes by warp shuffles: no barrier, and shared
 // memory only for the rows staged ahead.  The arithmetic is the tiled
 // sweep's, in the same order.
-// Euler's rows are staged like the marching strips' (kMAhead in flight), in
+// The rows are staged like the marching strips' (kMAhead in flight), in
 // a ring of kSSlots slots per lane: the slot refilled at row r is the one
-// read at row r - 1 (x sweep 0.255 -> 0.241 ms at 4096^2; the kernel had
-// waited on its one-row register prefetch).  Allaire's x sweep is bound by
-// instruction issue rather than load latency, and the staging instructions
-// made it 4 % slower, so it prefetches the next row into registers.
-template <int MODEL>
-__host__ __device__ constexpr bool seg_staged() {
-    return MODEL == MODEL_EULER;
-}
+// read at row r - 1.
 constexpr int kSSlots = kMAhead + 1;
 template <int MODEL>
 __host__ __device__ constexpr int seg_smem_bytes() {
-    return seg_staged<MODEL>() ? 4 * kSSlots * march_units<MODEL>() * 32 * 16 : 0;  // 4 warps per CTA
+    return 4 * kSSlots * march_units<MODEL>() * 32 * 16;  // 4 warps per CTA
 }
 constexpr int kSegCells = 28;  // outputs per row segment
 // rows of a tile: chosen per launch on the host (kSegMinRows..kSegRows) so
@@ -441,20 +435,22 @@ __device__ __forceinline__ void shfl_down_n(const float* x, float* y) {
     for (int q = 0; q < N; ++q) y[q] = __shfl_down_sync(0xffffffffu, x[q], 1);
 }
 
-template <int MODEL>
+template <int MODEL, int OPT>
 __device__ __forceinline__ void segment_tile(const MixedArgs& A, const TileGeom& g) {
     using MT = ModelTraits<MODEL>;
     constexpr int NV = MT::NV;
     const int lane = threadIdx.x & 31;
     const Inst& I = A.insts[g.inst];
-    const MPar P = load_par(I);
+    MPar P = load_par(I);
+    const bool wall_lo = (P.flags >> 5) & 1, wall_hi = (P.flags >> 6) & 1;  // left, right
+    if (OPT != kOptGeneral) P.flags = OPT;
     const double dt = I.st->dt;
     const float s_half = (float)(0.5 * (dt / I.dx));
     const float k_upd = (float)(dt / I.dx);
     const int nx = g.len, ny = g.wid;
     const int bin = g.cur, bout = g.cur ^ 1;
     const MPlanes qin = mplanes<MODEL>(I, bin), qout = mplanes<MODEL>(I, bout);
-    const long long pitch = I.pitch;
+    const unsigned pitch = I.pitch;
     const bool god = P.godunov();
     const int lim = P.limiter();
     // this lane's column and its mirrored source (pre_sweep's fill)
@@ -463,49 +459,36 @@ __device__ __forceinline__ void segment_tile(const MixedArgs& A, const TileGeom&
     bool neg = false;
     if (ga < 0) {
         src = -ga - 1;
-        neg = (P.flags >> 5) & 1;
+        neg = wall_lo;
     } else if (ga >= nx) {
         src = 2 * nx - 1 - ga;
-        neg = (P.flags >> 6) & 1;
+        neg = wall_hi;
     }
     src = min(max(src, 0), nx - 1);
     const bool writer = lane >= 2 && lane < 2 + kSegCells && ga < nx;
     const int row_end = min(g.b_org + A.rows, ny);
 
-    constexpr bool staged = seg_staged<MODEL>();
     extern __shared__ __align__(16) char seg_stage[];
     constexpr int MU = march_units<MODEL>();
-    char* stg = seg_stage + (threadIdx.x >> 5) * (kSSlots * MU * 32 * 16) + 16 * lane;
-    float nh[NV], nl[NV];  // the next row (unstaged form)
-    if constexpr (staged) {
+    constexpr int SB = MU * 32 * 16;
+    static_assert((kSSlots & (kSSlots - 1)) == 0, "a power of two");
+    char* stg = seg_stage + (threadIdx.x >> 5) * (kSSlots * SB) + 16 * lane;
+    unsigned off_in = (unsigned)g.b_org * pitch + src;           // the next row to load
+    unsigned off_out = (unsigned)g.b_org * pitch + (unsigned)ga;  // this row's cell
 #pragma unroll
-        for (int j = 0; j < kMAhead; ++j) {
-            if (g.b_org + j < row_end)
-                mstage_issue<MODEL>(stg, j, qin, (long long)(g.b_org + j) * pitch + src);
-            cp_async_commit();
-        }
-    } else {
-        load_cell<MODEL>(qin, (long long)g.b_org * pitch + src, nh, nl);
+    for (int j = 0; j < kMAhead; ++j) {
+        if (g.b_org + j < row_end) mstage_issue<MODEL>(stg + j * SB, qin, off_in);
+        off_in += pitch;
+        cp_async_commit();
     }
-    int slot = 0;
-    for (int row = g.b_org; row < row_end; ++row) {
+    int at = 0;
+    for (int row = g.b_org; row < row_end; ++row, off_in += pitch, off_out += pitch, ++at) {
         float h[NV], l[NV];
-        if constexpr (staged) {
-            asm volatile("cp.async.wait_group %0;\n" ::"n"(kMAhead - 1) : "memory");
-            mstage_read<MODEL>(stg, slot, h, l);
-            if (row + kMAhead < row_end)
-                mstage_issue<MODEL>(stg, slot == 0 ? kSSlots - 1 : slot - 1, qin,
-                                    (long long)(row + kMAhead) * pitch + src);
-            cp_async_commit();
-            slot = slot == kSSlots - 1 ? 0 : slot + 1;
-        } else {
-#pragma unroll
-            for (int q = 0; q < NV; ++q) {
-                h[q] = nh[q];
-                l[q] = nl[q];
-            }
-            if (row + 1 < row_end) load_cell<MODEL>(qin, (long long)(row + 1) * pitch + src, nh, nl);
-        }
+        asm volatile("cp.async.wait_group %0;\n" ::"n"(kMAhead - 1) : "memory");
+        mstage_read<MODEL>(stg + (unsigned)(at & (kSSlots - 1)) * SB, h, l);
+        if (row + kMAhead < row_end)
+            mstage_issue<MODEL>(stg + (unsigned)((at + kMAhead) & (kSSlots - 1)) * SB, qin, off_in);
+        cp_async_commit();
         if (neg) {
             h[MT::IM] = -h[MT::IM];
             l[MT::IM] = -l[MT::IM];
@@ -517,23 +500,11 @@ __device__ __forceinline__ void segment_tile(const MixedArgs& A, const TileGeom&
 
         // slopes and evolved face states of this cell (used by lanes 1..30)
         float Pf[NV], Mf[NV];
-        unsigned fl = 0;
+        bool okp = false, okm = false;
         if (!god) {
-            float d[NV], X[NV];
+            float d[NV];
             limit_all<NV>(lim, Wl, W, Wr, d);
-#pragma unroll
-            for (int q = 0; q < NV; ++q) Pf[q] = W[q] + 0.5f * d[q];
-            if (phys_prim<MODEL>(P, Pf)) fl |= 1u;
-#pragma unroll
-            for (int q = 0; q < NV; ++q) Pf[q] = W[q] - 0.5f * d[q];
-            if (phys_prim<MODEL>(P, Pf)) fl |= 2u;
-            jac_f<MODEL>(P, W, d, s_half, X);
-#pragma unroll
-            for (int q = 0; q < NV; ++q) Pf[q] = (W[q] + 0.5f * d[q]) - X[q];
-            if (phys_prim<MODEL>(P, Pf)) fl |= 4u;
-#pragma unroll
-            for (int q = 0; q < NV; ++q) Mf[q] = (W[q] - 0.5f * d[q]) - X[q];
-            if (phys_prim<MODEL>(P, Mf)) fl |= 8u;
+            face_states<MODEL>(P, W, d, s_half, Pf, Mf, okp, okm);
         } else {
 #pragma unroll
             for (int q = 0; q < NV; ++q) Pf[q] = Mf[q] = W[q];
@@ -542,11 +513,11 @@ __device__ __forceinline__ void segment_tile(const MixedArgs& A, const TileGeom&
         // HLLC at this cell's low face (between the lane below and this one)
         float PL[NV];
         shfl_up_n<NV>(Pf, PL);
-        const unsigned flL = __shfl_up_sync(0xffffffffu, fl, 1);
+        const unsigned okL = __ballot_sync(0xffffffffu, okp) << 1;  // bit l: lane l - 1
         float F[NV + 2];
         {
             float WL[NV], WR[NV];
-            const bool second = !god && (flL & 1u) && (fl & 2u) && (flL & 4u) && (fl & 8u);
+            const bool second = ((okL >> lane) & 1u) && okm;  // else first order
 #pragma unroll
             for (int q = 0; q < NV; ++q) {
                 WL[q] = second ? PL[q] : Wl[q];
@@ -558,11 +529,7 @@ __device__ __forceinline__ void segment_tile(const MixedArgs& A, const TileGeom&
         shfl_down_n<MODEL == MODEL_EULER ? NV : NV + 2>(F, FR);
 
         // compensated update (lanes 2 .. 2 + kSegCells - 1)
-#pragma unroll
-        for (int q = 0; q < NV; ++q) {
-            if (MODEL == MODEL_ALLAIRE && q == 5) continue;
-            comp_add(h[q], l[q], k_upd * (F[q] - FR[q]));
-        }
+        comp_update<NV>(h, l, k_upd, F, FR);
         if constexpr (MODEL == MODEL_ALLAIRE) {
             const float usL = F[NV], usR = FR[NV], zsL = F[NV + 1], zsR = FR[NV + 1];
             const float z = h[5];
@@ -577,12 +544,16 @@ __device__ __forceinline__ void segment_tile(const MixedArgs& A, const TileGeom&
             if (h[1] < 0.0f) { h[1] = 0.0f; l[1] = 0.0f; }
         }
         if constexpr (MODEL == MODEL_EULER) {
-            float Wn[NV];
-            c2p_mixed<MODEL>(I, P, h, l, Wn);
             // density / energy restore as in the plain form (rare)
-            if (writer && (!(h[0] > 1e-12f) || !(Wn[3] + P.gp1 > 0.0f))) {
+            float Wn[NV];
+            bool restore = writer && !euler_sure(h);
+            if (restore) {
+                c2p_mixed<MODEL>(I, P, h, l, Wn);
+                restore = !(h[0] > 1e-12f) || !(Wn[3] + P.gp1 > 0.0f);
+            }
+            if (restore) {
                 float oh[NV], ol[NV], Wo[NV];  // the cell before the update
-                load_cell<MODEL>(qin, (long long)row * pitch + src, oh, ol);
+                load_cell<MODEL>(qin, (unsigned)row * pitch + src, oh, ol);
                 c2p_mixed<MODEL>(I, P, oh, ol, Wo);
                 float rho = h[0] > 1e-12f ? h[0] : oh[0];
                 float u = Wn[1], v = Wn[2];
@@ -593,22 +564,32 @@ __device__ __forceinline__ void segment_tile(const MixedArgs& A, const TileGeom&
                 h[3] = (p + P.gp1) * P.i1 + 0.5f * rho * (u * u + v * v); l[3] = 0.f;
             }
         }
-        if (writer) store_cell<MODEL>(qout, (long long)row * pitch + ga, h, l);
+        if (writer) store_cell<MODEL>(qout, off_out, h, l);
     }
 }
 
 // Persistent x sweep: warp w of the W warps of the grid walks the tiles w,
-// w + W, w + 2W, ... of the launch's tile list.  Euler is bounded to 64
-// registers for 8 CTAs per SM (8 % faster than 7 CTAs when the next row was
-// still prefetched into registers); Allaire is fastest unbounded.
-template <int MODEL>
-__global__ void __launch_bounds__(128, MODEL == MODEL_EULER ? 8 : 1)
+// w + W, w + 2W, ... of the launch's tile list.  Bounded to 64 (Euler) and 96
+// (Allaire) registers for 8 and 5 CTAs per SM.
+//
+// Both sweeps are bound by instruction issue: at 2048^2 Euler the x sweep runs
+// 286 thread instructions a cell (74 % of the issue slots, 5.4 TB/s of its
+// 268 MB, 82 % of the measured copy) and the y sweep 286 (69 %, 4.2 TB/s),
+// against 384 and 390 before the slopes, face states and sums went through
+// pairs of components, minmod took three instructions, one reciprocal served
+// both star quotients, the physicality tests were made on the smallest values
+// and the options were fixed at compile time: x 66.2 -> 49.8 us, y 80.4 ->
+// 63.9 us a sweep.  Allaire at 2048x1024: x 62.7 -> 45.9 us, y 84.8 -> 68.1 us
+// (x with its rows staged and 5 CTAs per SM instead of the next row in
+// registers and 4: 49.1 -> 45.9).
+template <int MODEL, int OPT>
+__global__ void __launch_bounds__(128, MODEL == MODEL_EULER ? 8 : 5)
     mixed_segment_x_kernel(MixedArgs A) {
     const int gw = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int nw = gridDim.x * (blockDim.x >> 5);
     for (int tile = gw; tile < A.ntiles; tile += nw) {
         const TileGeom g = tile_geom<DIR_X, kSegCells, kSegRows>(A, tile);
-        if (!g.skip) segment_tile<MODEL>(A, g);
+        if (!g.skip) segment_tile<MODEL, OPT>(A, g);
     }
 }
 

@@ -48,6 +48,7 @@ struct Inst {
     // FP32 constants of the sweeps (loaded into registers once per tile):
     // g1, p1, g1 - 1, g1 p1, 1/(g1 - 1), 1/(g2 - 1), g1 p1/(g1 - 1), g2 p2/(g2 - 1)
     alignas(16) float pf[8];
+    alignas(16) float zf[4];  // z_min and 1 - z_min as value + compensation word
     int flags;       // limiter (bits 0-1), PVRS speeds (2), Godunov (3), stiffened gas (4),
                      // reflective walls L, R, B, T (5-8)
     // FP64 mixture constants for the pressure of stiffened-gas cells:
@@ -113,6 +114,15 @@ __device__ __forceinline__ void cp_async8(void* smem_dst, const void* gsrc) {
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_group 0;\n" ::: "memory"); }
 
+// FP64 -> FP32 by the conversion alone (with -ftz the cast also tests and
+// flushes the result: two more instructions; the results here are pressures,
+// densities and steps, far from FP32's denormals, and the FP32 operations on
+// them flush one anyway).
+__device__ __forceinline__ float to_float(double x) {
+    float r;
+    asm("cvt.rn.f32.f64 %0, %1;" : "=f"(r) : "d"(x));
+    return r;
+}
 __device__ __forceinline__ float frcp(float x) { return 1.0f / x; }
 // Approximate quotient without the operand range scaling of `a / b` (which
 // only matters for |b| > 2^126; every divisor here, a density, a pressure,
@@ -120,15 +130,72 @@ __device__ __forceinline__ float frcp(float x) { return 1.0f / x; }
 // Measured 3-4 % faster on the sweeps, the same results on every test case.
 __device__ __forceinline__ float fdiv(float a, float b) { return __fdividef(a, b); }
 __device__ __forceinline__ float fsqrt(float x) { return sqrtf(x); }
-__device__ __forceinline__ float fminf_s(float a, float b) { return (b < a) ? b : a; }
-__device__ __forceinline__ float fmaxf_s(float a, float b) { return (a < b) ? b : a; }
+// One instruction each (the comparison forms of the reference's std::min and
+// std::max take two); a NaN operand gives the other one.
+__device__ __forceinline__ float fminf_s(float a, float b) { return fminf(a, b); }
+__device__ __forceinline__ float fmaxf_s(float a, float b) { return fmaxf(a, b); }
+
+// The same giving NaN for a NaN operand, for tests that a NaN has to fail.
+__device__ __forceinline__ float fmin_n(float a, float b) {
+    float r;
+    asm("min.NaN.ftz.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ float fmax_n(float a, float b) {
+    float r;
+    asm("max.NaN.ftz.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
+    return r;
+}
+
+// Two FP32 values in one 64-bit register pair: sm_100 adds, multiplies and
+// fuses both with one instruction, each rounded as the scalar instruction
+// rounds it.  The sweeps are bound by instruction issue, so the component-wise
+// parts of the update (slope differences, face states, the compensated sum)
+// go through pairs of components.
+struct F2 {
+    unsigned long long v;
+};
+__device__ __forceinline__ F2 f2(float a, float b) {
+    F2 r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r.v) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ void f2_get(F2 x, float& a, float& b) {
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(x.v));
+}
+__device__ __forceinline__ F2 add2(F2 a, F2 b) {
+    F2 r;
+    asm("add.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 sub2(F2 a, F2 b) {
+    F2 r;
+    asm("sub.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 mul2(F2 a, F2 b) {
+    F2 r;
+    asm("mul.rn.ftz.f32x2 %0, %1, %2;" : "=l"(r.v) : "l"(a.v), "l"(b.v));
+    return r;
+}
+__device__ __forceinline__ F2 fma2(F2 a, F2 b, F2 c) {
+    F2 r;
+    asm("fma.rn.ftz.f32x2 %0, %1, %2, %3;" : "=l"(r.v) : "l"(a.v), "l"(b.v), "l"(c.v));
+    return r;
+}
+// y = x over N (even) components, by pairs.
+template <int N, class Fn>
+__device__ __forceinline__ void pairs(Fn fn) {
+#pragma unroll
+    for (int q = 0; q < N; q += 2) fn(q);
+}
 
 // Mixture coefficients eps(z) = z/(g1-1) + (1-z)/(g2-1) and
-// k(z) = (z g1 p1/(g1-1) + (1-z) g2 p2/(g2-1)) / eps in FP32.
-__device__ __forceinline__ void mix_f(const MPar& P, float z, float& eps, float& k) {
-    float omz = 1.0f - z;
+// eps k(z) = z g1 p1/(g1-1) + (1-z) g2 p2/(g2-1) in FP32.
+__device__ __forceinline__ void mix_f(const MPar& P, float z, float& eps, float& kn) {
+    const float omz = 1.0f - z;
     eps = z * P.i1 + omz * P.i2;
-    k = (z * P.c1 + omz * P.c2) * frcp(eps);
+    kn = z * P.c1 + omz * P.c2;
 }
 
 // Primitive state (rho-split for Allaire: W = rho1 z, rho2 (1-z), u, v, p, z).
@@ -153,7 +220,7 @@ __device__ __forceinline__ void c2p_mixed(const Inst& I, const MPar& P, const fl
             double M1 = (double)hi[1] + (double)lo[1], M2 = (double)hi[2] + (double)lo[2];
             double E = (double)hi[3] + (double)lo[3];
             double re = E - 0.5 * (M1 * M1 + M2 * M2) / R;
-            p = (float)(__ldg(&I.eos.gm1_1) * re - __ldg(&I.eos.gp1));
+            p = to_float(__ldg(&I.eos.gm1_1) * re - __ldg(&I.eos.gp1));
         }
         W[0] = rho;
         W[1] = u;
@@ -180,7 +247,7 @@ __device__ __forceinline__ void c2p_mixed(const Inst& I, const MPar& P, const fl
             double omz = 1.0 - zz;
             double eps = zz * __ldg(I.pd + 0) + omz * __ldg(I.pd + 1);
             double kn = zz * __ldg(I.pd + 2) + omz * __ldg(I.pd + 3);
-            p = fdiv((float)((E * R - 0.5 * (M1 * M1 + M2 * M2)) - kn * R), (float)(R * eps));
+            p = fdiv(to_float((E * R - 0.5 * (M1 * M1 + M2 * M2)) - kn * R), to_float(R * eps));
         }
         W[0] = hi[0];
         W[1] = hi[1];
@@ -211,18 +278,25 @@ template <int MODEL> __device__ __forceinline__ bool phys_prim(const MPar& P, co
     }
 }
 
+// The median of a, b and 0: minmod (the smaller in size where the signs
+// agree, else 0) in three instructions: the smaller size with the product's
+// sign, clipped at 0, under the sign of a.
+__device__ __forceinline__ float median0(float a, float b) {
+    float x;
+    asm("min.ftz.xorsign.abs.f32 %0, %1, %2;" : "=f"(x) : "f"(a), "f"(b));
+    return __int_as_float(__float_as_int(fmaxf(x, 0.0f)) | (__float_as_int(a) & 0x80000000));
+}
+
 __device__ __forceinline__ float limit_f(int lim, float a, float b) {
     switch (lim) {
         case LIM_VANLEER:
             return (a * b > 0.0f) ? fdiv(2.0f * a * b, a + b) : 0.0f;
         case LIM_MC:
-            if (b >= 0.0f && a >= 0.0f) return fminf_s(0.5f * (a + b), fminf_s(2.0f * a, 2.0f * b));
-            if (b <= 0.0f && a <= 0.0f) return fmaxf_s(0.5f * (a + b), fmaxf_s(2.0f * a, 2.0f * b));
-            return 0.0f;
+            return median0(0.5f * (a + b), 2.0f * median0(a, b));
         case LIM_UNLIMITED:
             return 0.5f * (a + b);
         default:
-            return (b > 0.0f) ? fmaxf_s(0.0f, fminf_s(a, b)) : fminf_s(0.0f, fmaxf_s(a, b));
+            return median0(a, b);
     }
 }
 
@@ -231,22 +305,28 @@ __device__ __forceinline__ float limit_f(int lim, float a, float b) {
 template <int NV>
 __device__ __forceinline__ void limit_all(int lim, const float* Wm, const float* W, const float* Wp,
                                           float* d) {
+    float a[NV], b[NV];
+    pairs<NV>([&](int q) {
+        const F2 w = f2(W[q], W[q + 1]);
+        f2_get(sub2(w, f2(Wm[q], Wm[q + 1])), a[q], a[q + 1]);
+        f2_get(sub2(f2(Wp[q], Wp[q + 1]), w), b[q], b[q + 1]);
+    });
     switch (lim) {
         case LIM_VANLEER:
 #pragma unroll
-            for (int q = 0; q < NV; ++q) d[q] = limit_f(LIM_VANLEER, W[q] - Wm[q], Wp[q] - W[q]);
+            for (int q = 0; q < NV; ++q) d[q] = limit_f(LIM_VANLEER, a[q], b[q]);
             break;
         case LIM_MC:
 #pragma unroll
-            for (int q = 0; q < NV; ++q) d[q] = limit_f(LIM_MC, W[q] - Wm[q], Wp[q] - W[q]);
+            for (int q = 0; q < NV; ++q) d[q] = limit_f(LIM_MC, a[q], b[q]);
             break;
         case LIM_UNLIMITED:
 #pragma unroll
-            for (int q = 0; q < NV; ++q) d[q] = limit_f(LIM_UNLIMITED, W[q] - Wm[q], Wp[q] - W[q]);
+            for (int q = 0; q < NV; ++q) d[q] = limit_f(LIM_UNLIMITED, a[q], b[q]);
             break;
         default:
 #pragma unroll
-            for (int q = 0; q < NV; ++q) d[q] = limit_f(LIM_MINMOD, W[q] - Wm[q], Wp[q] - W[q]);
+            for (int q = 0; q < NV; ++q) d[q] = limit_f(LIM_MINMOD, a[q], b[q]);
     }
 }
 
@@ -263,122 +343,152 @@ template <int MODEL> __device__ __forceinline__ float sound_f(const MPar& P, con
     }
 }
 
-// Half-step evolution X = (0.5 dt/dx) A(W) d (primitive Jacobian).
+// Half-step evolution X = (0.5 dt/dx) A(W) d (primitive Jacobian), rho c^2
+// without the root and the division by rho that c itself would take.
 template <int MODEL>
 __device__ __forceinline__ void jac_f(const MPar& P, const float* W, const float* d, float s,
                                       float* X) {
-    float c = sound_f<MODEL>(P, W);
     if constexpr (MODEL == MODEL_EULER) {
-        float rho = W[0], u = W[1];
+        const float rho = W[0], u = W[1];
+        const float rc2 = fmaxf(0.0f, P.g1 * (W[3] + P.p1));
         X[0] = s * (u * d[0] + rho * d[1]);
         X[1] = s * (u * d[1] + frcp(rho) * d[3]);
         X[2] = s * (u * d[2]);
-        X[3] = s * (rho * c * c * d[1] + u * d[3]);
+        X[3] = s * (rc2 * d[1] + u * d[3]);
     } else {
-        float rho = W[0] + W[1], u = W[2];
+        const float rho = W[0] + W[1], u = W[2];
+        float eps, kn;
+        mix_f(P, W[5], eps, kn);
+        const float rc2 = fmaxf(0.0f, fdiv(kn + W[4] * (1.0f + eps), eps));
         X[0] = s * (u * d[0] + W[0] * d[2]);
         X[1] = s * (u * d[1] + W[1] * d[2]);
         X[2] = s * (u * d[2] + frcp(rho) * d[4]);
         X[3] = s * (u * d[3]);
-        X[4] = s * (rho * c * c * d[2] + u * d[4]);
+        X[4] = s * (rc2 * d[2] + u * d[4]);
         X[5] = s * (u * d[5]);
     }
 }
 
+// Evolved face states of a cell, Wp (high face) and Wm (low face), from its
+// slopes d, and whether the reference would use them: each needs its
+// slope-extrapolated state and its evolved state physical
+// (E/headers/flux_solver_MUSCLhancock.hpp:178-223).  Where the smallest
+// values of all four states pass, all pass; only otherwise are they tested one
+// by one (for the mixture a pressure >= 0 is sufficient, eps k being >= 0).
+template <int MODEL>
+__device__ __forceinline__ void face_states(const MPar& P, const float* W, const float* d, float s,
+                                            float* Wp, float* Wm, bool& okp, bool& okm) {
+    constexpr int NV = ModelTraits<MODEL>::NV;
+    float E[NV], D[NV], X[NV];  // slope-extrapolated states (high, low), half step
+    jac_f<MODEL>(P, W, d, s, X);
+    const F2 half = f2(0.5f, 0.5f), mhalf = f2(-0.5f, -0.5f);
+    pairs<NV>([&](int q) {
+        const F2 w = f2(W[q], W[q + 1]), dq = f2(d[q], d[q + 1]), x = f2(X[q], X[q + 1]);
+        const F2 e = fma2(half, dq, w), m = fma2(mhalf, dq, w);
+        f2_get(e, E[q], E[q + 1]);
+        f2_get(m, D[q], D[q + 1]);
+        f2_get(sub2(e, x), Wp[q], Wp[q + 1]);
+        f2_get(sub2(m, x), Wm[q], Wm[q + 1]);
+    });
+    bool all;
+    auto least = [&](int q) {  // the smallest of component q over the four states
+        return fmin_n(fmin_n(E[q], D[q]), fmin_n(Wp[q], Wm[q]));
+    };
+    if constexpr (MODEL == MODEL_EULER) {
+        all = (least(0) > 0.0f) & (least(3) + P.gp1 >= 0.0f);
+    } else {
+        const float zm = fmax_n(fmax_n(E[5], D[5]), fmax_n(Wp[5], Wm[5]));
+        const float r1 = least(0), r2 = least(1);
+        all = (fmin_n(fmin_n(r1, r2), fmin_n(least(4), least(5))) >= 0.0f) & (zm <= 1.0f) &
+              (r1 + r2 > 0.0f);
+    }
+    okp = okm = all;
+    if (!all) {
+        okp = phys_prim<MODEL>(P, E) && phys_prim<MODEL>(P, Wp);
+        okm = phys_prim<MODEL>(P, D) && phys_prim<MODEL>(P, Wm);
+    }
+}
+
 // HLLC flux from primitive face states (same wave-speed estimates and star
-// states as hllc_flux in cfd_physics.cuh).  F[NV] = flux, F[NV] = u*,
-// F[NV+1] = z* (Allaire).
+// states as hllc_flux in cfd_physics.cuh), F[NV] = u*, F[NV+1] = z* (Allaire).
+// With the star factor f = (S - u)/(S - u*), the passive components' flux
+// U u + w (f U - U) is U A with A = u + w (f - 1), w the selected wave speed
+// clipped at 0, and p/(S - u) enters the energy as f p/(S - u) = p/(S - u*),
+// so one reciprocal serves both.
 template <int MODEL>
 __device__ __forceinline__ void hllc_prim(const MPar& P, const float* WL, const float* WR,
                                           float* F) {
     using T = ModelTraits<MODEL>;
     constexpr int NV = T::NV;
-    float rL, rR, uL, uR, pL, pR, cL, cR, epsL = 1.f, kL = 0.f, epsR = 1.f, kR = 0.f;
+    float rL, rR, uL, uR, pL, pR, cL, cR, epsL = 1.f, knL = 0.f, epsR = 1.f, knR = 0.f;
+    float qL = 0.f, qR = 0.f;  // 1/(eps rho)
     if constexpr (MODEL == MODEL_EULER) {
         rL = WL[0]; uL = WL[1]; pL = WL[3];
         rR = WR[0]; uR = WR[1]; pR = WR[3];
-        cL = fsqrt(fmaxf_s(0.0f, fdiv(P.g1 * (pL + P.p1), rL)));
-        cR = fsqrt(fmaxf_s(0.0f, fdiv(P.g1 * (pR + P.p1), rR)));
+        cL = fsqrt(fmaxf(0.0f, fdiv(P.g1 * (pL + P.p1), rL)));
+        cR = fsqrt(fmaxf(0.0f, fdiv(P.g1 * (pR + P.p1), rR)));
     } else {
         rL = WL[0] + WL[1]; uL = WL[2]; pL = WL[4];
         rR = WR[0] + WR[1]; uR = WR[2]; pR = WR[4];
-        mix_f(P, WL[5], epsL, kL);
-        mix_f(P, WR[5], epsR, kR);
-        cL = fsqrt(fmaxf_s(0.0f, fdiv(kL + pL * (frcp(epsL) + 1.0f), rL)));
-        cR = fsqrt(fmaxf_s(0.0f, fdiv(kR + pR * (frcp(epsR) + 1.0f), rR)));
+        mix_f(P, WL[5], epsL, knL);
+        mix_f(P, WR[5], epsR, knR);
+        qL = frcp(epsL * rL);
+        qR = frcp(epsR * rR);
+        cL = fsqrt(fmaxf(0.0f, (knL + pL * (1.0f + epsL)) * qL));
+        cR = fsqrt(fmaxf(0.0f, (knR + pR * (1.0f + epsR)) * qR));
     }
     float SL, SR;
     if (MODEL == MODEL_ALLAIRE && P.pvrs()) {
-        float ra = 0.5f * (rL + rR), ca = 0.5f * (cL + cR);
-        float ppv = fmaxf_s(0.0f, 0.5f * (pL + pR) + 0.5f * (uL - uR) * ra * ca);
-        if (ppv > pL) {
-            float pa = 0.5f * (ppv + pL);
-            SL = uL - fsqrt(fmaxf_s(0.0f, fdiv(ppv + kL + fdiv(pa, epsL), rL)));
-        } else {
-            SL = uL - cL;
-        }
-        if (ppv > pR) {
-            float pa = 0.5f * (ppv + pR);
-            SR = uR + fsqrt(fmaxf_s(0.0f, fdiv(ppv + kR + fdiv(pa, epsR), rR)));
-        } else {
-            SR = uR + cR;
-        }
+        const float ra = 0.5f * (rL + rR), ca = 0.5f * (cL + cR);
+        const float ppv = fmaxf(0.0f, 0.5f * (pL + pR) + 0.5f * (uL - uR) * ra * ca);
+        // shock_speed_jump: sqrt(((p* + k) + ((p* + p)/2)/eps) / rho)
+        SL = uL - (ppv > pL ? fsqrt(fmaxf(0.0f, (knL + ppv * epsL + 0.5f * (ppv + pL)) * qL)) : cL);
+        SR = uR + (ppv > pR ? fsqrt(fmaxf(0.0f, (knR + ppv * epsR + 0.5f * (ppv + pR)) * qR)) : cR);
     } else {
-        float ua = 0.5f * (uL + uR), ca = 0.5f * (cL + cR);
-        SL = fminf_s(ua - ca, uL - cL);
-        SR = fmaxf_s(ua + ca, uR + cR);
+        const float ua = 0.5f * (uL + uR), ca = 0.5f * (cL + cR);
+        SL = fminf(ua - ca, uL - cL);
+        SR = fmaxf(ua + ca, uR + cR);
     }
-    float dSL = SL - uL, dSR = SR - uR;
-    float us = fdiv((pR - pL) + rL * uL * dSL - rR * uR * dSR, rL * dSL - rR * dSR);
-    bool left = !signbit(us);
+    const float dSL = SL - uL, dSR = SR - uR;
+    const float mL = rL * dSL, mR = rR * dSR;
+    const float us = fdiv((pR - pL) + mL * uL - mR * uR, mL - mR);
+    const bool left = !signbit(us);
     // per-element selects (a pointer to either side would put both in local memory)
-    float rho = left ? rL : rR, u = left ? uL : uR, p = left ? pL : pR;
-    float Sk = left ? SL : SR, dS = left ? dSL : dSR;
-    float wave = left ? fminf_s(0.0f, SL) : fmaxf_s(0.0f, SR);
-    float fac = fdiv(dS, Sk - us);
-    // conserved state of the selected side
-    float U[NV];
+    const float rho = left ? rL : rR, u = left ? uL : uR, p = left ? pL : pR;
+    const float Sk = left ? SL : SR, dS = left ? dSL : dSR;
+    const float wave = left ? fminf(0.0f, SL) : fmaxf(0.0f, SR);
+    const float v = left ? WL[T::IT] : WR[T::IT];
+    const float inv = frcp(Sk - us);
+    const float fac = dS * inv;
+    const float A = u + wave * (fac - 1.0f);
+    float re;  // rho e
     if constexpr (MODEL == MODEL_EULER) {
-        float v = left ? WL[2] : WR[2];
-        U[0] = rho;
-        U[1] = rho * u;
-        U[2] = rho * v;
-        U[3] = (p + P.gp1) * P.i1 + 0.5f * rho * (u * u + v * v);
+        re = (p + P.gp1) * P.i1;
     } else {
-        float v = left ? WL[3] : WR[3];
-        float eps = left ? epsL : epsR, k = left ? kL : kR;
-        U[0] = left ? WL[0] : WR[0];
-        U[1] = left ? WL[1] : WR[1];
-        U[2] = rho * u;
-        U[3] = rho * v;
-        U[4] = (p + k) * eps + 0.5f * rho * (u * u + v * v);
-        U[5] = left ? WL[5] : WR[5];
+        const float eps = left ? epsL : epsR, kn = left ? knL : knR;
+        re = p * eps + kn;
     }
-    float Us[NV];
-#pragma unroll
-    for (int k = 0; k < NV; ++k) Us[k] = fac * U[k];
-    Us[T::IM] = fac * rho * us;
-    Us[T::IE] = fac * (U[T::IE] + (us - u) * (rho * us + fdiv(p, dS)));
-    float Fp[NV];
+    const float E = re + 0.5f * rho * (u * u + v * v);
+    const float m = rho * A;
     if constexpr (MODEL == MODEL_EULER) {
-        Fp[0] = U[0] * u;
-        Fp[1] = U[1] * u + p;
-        Fp[2] = U[2] * u;
-        Fp[3] = (U[3] + p) * u;
+        F[0] = m;
     } else {
-        Fp[0] = U[0] * u;
-        Fp[1] = U[1] * u;
-        Fp[2] = U[2] * u + p;
-        Fp[3] = U[3] * u;
-        Fp[4] = (U[4] + p) * u;
-        Fp[5] = 0.0f;
-        Us[5] = U[5];
+        F[0] = (left ? WL[0] : WR[0]) * A;
+        F[1] = (left ? WL[1] : WR[1]) * A;
+        F[5] = 0.0f;
     }
-#pragma unroll
-    for (int k = 0; k < NV; ++k) F[k] = Fp[k] + wave * (Us[k] - U[k]);
-    if constexpr (MODEL == MODEL_ALLAIRE) F[5] = 0.0f;
+    F[T::IM] = rho * (u * u + wave * (fac * us - u)) + p;
+    F[T::IT] = m * v;
+    F[T::IE] = E * A + p * u + (wave * (us - u)) * (fac * rho * us + p * inv);
     F[NV] = us;
     if constexpr (MODEL == MODEL_ALLAIRE) F[NV + 1] = left ? WL[5] : WR[5];
+}
+
+// Whether an updated Euler state is sure to keep rho > 0 and rho e > 0
+// (p + gamma p_inf > 0): rho E clears |m|^2/2 by more than its rounding.
+// Otherwise the caller converts the state and tests it as the reference does.
+__device__ __forceinline__ bool euler_sure(const float* h) {
+    return (h[0] > 1e-12f) & (h[0] * h[3] > 0.500001f * (h[1] * h[1] + h[2] * h[2]));
 }
 
 // hi + lo += d with an error-free transformation (TwoSum), keeping the pair
@@ -390,6 +500,30 @@ __device__ __forceinline__ void comp_add(float& hi, float& lo, float d) {
     float e = (hi - (s - bp)) + (y - bp);
     hi = s;
     lo = e;
+}
+
+// The same for a pair, d = k (a - b).
+__device__ __forceinline__ void comp_add2(float* hi, float* lo, F2 k, F2 a, F2 b) {
+    const F2 h = f2(hi[0], hi[1]);
+    const F2 y = fma2(k, sub2(a, b), f2(lo[0], lo[1]));
+    const F2 s = add2(h, y);
+    const F2 bp = sub2(s, h);
+    const F2 e = add2(sub2(h, sub2(s, bp)), sub2(y, bp));
+    f2_get(s, hi[0], hi[1]);
+    f2_get(e, lo[0], lo[1]);
+}
+// The conservative update of a cell from the fluxes at its two faces (all
+// components; the caller sets Allaire's z, whose flux is 0).
+template <int NV>
+__device__ __forceinline__ void comp_update(float* h, float* l, float k, const float* FL, const float* FR) {
+    const F2 kk = f2(k, k);
+    pairs<NV>([&](int q) {
+        if (NV == 6 && q == 4) {  // E alone: z has its own update
+            comp_add(h[4], l[4], k * (FL[4] - FR[4]));
+            return;
+        }
+        comp_add2(h + q, l + q, kk, f2(FL[q], FL[q + 1]), f2(FR[q], FR[q + 1]));
+    });
 }
 
 // The planes of one state buffer of a member, held in registers: the stores
@@ -411,8 +545,8 @@ __device__ __forceinline__ MPlanes mplanes(const Inst& I, int buf) {
     return q;
 }
 
-template <int MODEL> __device__ __forceinline__ void load_cell(const MPlanes& Q, long long off, float* h,
-                                                               float* l) {
+template <int MODEL, class Off>
+__device__ __forceinline__ void load_cell(const MPlanes& Q, Off off, float* h, float* l) {
     float4 a = __ldg(Q.v4 + off), b = __ldg(Q.c4 + off);
     h[0] = a.x; h[1] = a.y; h[2] = a.z; h[3] = a.w;
     l[0] = b.x; l[1] = b.y; l[2] = b.z; l[3] = b.w;
@@ -423,8 +557,8 @@ template <int MODEL> __device__ __forceinline__ void load_cell(const MPlanes& Q,
     }
 }
 
-template <int MODEL> __device__ __forceinline__ void store_cell(const MPlanes& Q, long long off,
-                                                                const float* h, const float* l) {
+template <int MODEL, class Off>
+__device__ __forceinline__ void store_cell(const MPlanes& Q, Off off, const float* h, const float* l) {
     Q.v4[off] = make_float4(h[0], h[1], h[2], h[3]);
     Q.c4[off] = make_float4(l[0], l[1], l[2], l[3]);
     if constexpr (MODEL == MODEL_ALLAIRE) {
@@ -441,10 +575,9 @@ template <int MODEL> __device__ __forceinline__ void load_cell(const Inst& I, in
 // The clip of the updated volume fraction to [z_min, 1 - z_min] on a
 // compensated z (value h, compensation l).
 __device__ __forceinline__ void clip_z(const Inst& I, float& h, float& l) {
-    const double zm = __ldg(&I.z_min);
-    const float zlo = (float)zm, zhi = (float)(1.0 - zm);
-    if (h + l < zlo) { h = zlo; l = (float)(zm - (double)zlo); }
-    if (h + l > zhi) { h = zhi; l = (float)((1.0 - zm) - (double)zhi); }
+    const float4 b = __ldg(reinterpret_cast<const float4*>(I.zf));
+    if (h + l < b.x) { h = b.x; l = b.y; }
+    if (h + l > b.z) { h = b.z; l = b.w; }
 }
 
 template <int MODEL> __device__ __forceinline__ void store_cell(const Inst& I, int buf,
@@ -645,28 +778,16 @@ __device__ __forceinline__ void mixed_tile(const MixedArgs& A, const TileGeom& g
         int a, b;
         Tl::item(tid, 1, LA - 2, a, b);
         int s = Tl::slot(a, b);
-        float W[NV], Wl[NV], Wr[NV], d[NV], X[NV], Wt[NV];
+        float W[NV], Wl[NV], Wr[NV], d[NV], Wp[NV], Wm[NV];
         sW.get(s, W);
         sW.get(s - ST, Wl);
         sW.get(s + ST, Wr);
         limit_all<NV>(P.limiter(), Wl, W, Wr, d);
-        unsigned fl = 0;
-#pragma unroll
-        for (int k = 0; k < NV; ++k) Wt[k] = W[k] + 0.5f * d[k];
-        if (phys_prim<MODEL>(P, Wt)) fl |= 1u;
-#pragma unroll
-        for (int k = 0; k < NV; ++k) Wt[k] = W[k] - 0.5f * d[k];
-        if (phys_prim<MODEL>(P, Wt)) fl |= 2u;
-        jac_f<MODEL>(P, W, d, s_half, X);
-#pragma unroll
-        for (int k = 0; k < NV; ++k) Wt[k] = (W[k] + 0.5f * d[k]) - X[k];
-        if (phys_prim<MODEL>(P, Wt)) fl |= 4u;
-        sP.put(s, Wt);
-#pragma unroll
-        for (int k = 0; k < NV; ++k) Wt[k] = (W[k] - 0.5f * d[k]) - X[k];
-        if (phys_prim<MODEL>(P, Wt)) fl |= 8u;
-        sM.put(s, Wt);
-        sFl[s] = (unsigned char)fl;
+        bool okp, okm;
+        face_states<MODEL>(P, W, d, s_half, Wp, Wm, okp, okm);
+        sP.put(s, Wp);
+        sM.put(s, Wm);
+        sFl[s] = (unsigned char)((okp ? 1 : 0) | (okm ? 2 : 0));
     }
     __syncthreads();
 
@@ -681,7 +802,7 @@ __device__ __forceinline__ void mixed_tile(const MixedArgs& A, const TileGeom& g
             unsigned fL = sFl[sL], fR = sFl[sR];
             // zero slopes evolve to the cell state itself; the first-order
             // fallback uses the cell states too
-            if ((fL & 1u) && (fR & 2u) && (fL & 4u) && (fR & 8u)) {
+            if ((fL & 1u) && (fR & 2u)) {
                 first = false;
                 sP.get(sL, WL);
                 sM.get(sR, WR);
@@ -714,11 +835,7 @@ __device__ __forceinline__ void mixed_tile(const MixedArgs& A, const TileGeom& g
                 float FL[NV], FR[NV];
                 sF.get(s, FL);
                 sF.get(s + ST, FR);
-#pragma unroll
-                for (int k = 0; k < NV; ++k) {
-                    if (MODEL == MODEL_ALLAIRE && k == 5) continue;
-                    comp_add(hh[k], ll[k], k_upd * (FL[k] - FR[k]));
-                }
+                comp_update<NV>(hh, ll, k_upd, FL, FR);
             }
             if constexpr (MODEL == MODEL_ALLAIRE) {
                 float2 uzL = sUZ[s], uzR = sUZ[s + ST];
