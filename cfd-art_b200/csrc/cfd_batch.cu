@@ -91,34 +91,47 @@ int launch_t(const MixedArgs& a, int sms, cudaStream_t st) {
     return CFD_OK;
 }
 
-// The warp sweeps of the mixed form (4-warp CTAs): marching y sweep, segment
-// x sweep, each for one set of options.
+// The warp sweeps (4-warp CTAs) of both forms: segment x sweep, marching y
+// sweep, each for one set of options.
 struct WarpKernel {
     void (*fn)(MixedArgs);
     int smem;
 };
 template <int MODEL, int OPT>
-WarpKernel warp_kernel(int dir) {
+WarpKernel warp_kernel(int fp64, int dir) {
+    if (fp64)
+        return dir == DIR_X
+                   ? WarpKernel{fast::fast_segment_x_kernel<MODEL, OPT>, fast::segment64_smem_bytes<MODEL>()}
+                   : WarpKernel{fast::fast_march_kernel<MODEL, OPT>, fast::march64_smem_bytes<MODEL>()};
     return dir == DIR_X ? WarpKernel{mixed_segment_x_kernel<MODEL, OPT>, seg_smem_bytes<MODEL>()}
                         : WarpKernel{mixed_march_kernel<MODEL, OPT>, march_smem_bytes<MODEL>()};
 }
-template <int MODEL>
-WarpKernel warp_kernel(int dir, int opt) {
-    if (opt == common_options<MODEL>(0)) return warp_kernel<MODEL, common_options<MODEL>(0)>(dir);
-    if (opt == common_options<MODEL>(1)) return warp_kernel<MODEL, common_options<MODEL>(1)>(dir);
-    return warp_kernel<MODEL, kOptGeneral>(dir);
-}
-WarpKernel warp_kernel(int model, int dir, int opt) {
-    return model == CFD_MODEL_EULER ? warp_kernel<MODEL_EULER>(dir, opt)
-                                    : warp_kernel<MODEL_ALLAIRE>(dir, opt);
+// The option sets compiled by themselves (a gas with each limiter or in first
+// order; water and gas with PVRS speeds, two gases); at 2048^2 Euler minmod the
+// instantiation takes 49.9 + 63.2 us (x + y) where the general mixed kernels,
+// the fall-back for every other set, take 55.1 + 73.5.
+WarpKernel warp_kernel(int model, int fp64, int dir, int opt) {
+    if (model == CFD_MODEL_EULER) switch (opt) {
+            case LIM_MINMOD: return warp_kernel<MODEL_EULER, LIM_MINMOD>(fp64, dir);
+            case LIM_VANLEER: return warp_kernel<MODEL_EULER, LIM_VANLEER>(fp64, dir);
+            case LIM_MC: return warp_kernel<MODEL_EULER, LIM_MC>(fp64, dir);
+            case MF_GODUNOV: return warp_kernel<MODEL_EULER, MF_GODUNOV>(fp64, dir);
+            default: return warp_kernel<MODEL_EULER, kOptGeneral>(fp64, dir);
+        }
+    switch (opt) {
+        case LIM_MINMOD | MF_PVRS | MF_STIFF:
+            return warp_kernel<MODEL_ALLAIRE, LIM_MINMOD | MF_PVRS | MF_STIFF>(fp64, dir);
+        case LIM_MINMOD: return warp_kernel<MODEL_ALLAIRE, LIM_MINMOD>(fp64, dir);
+        default: return warp_kernel<MODEL_ALLAIRE, kOptGeneral>(fp64, dir);
+    }
 }
 
 // Resident CTAs per SM of such a kernel.
-int warp_per_sm(int model, int dir, int opt) {
-    static int known[2][2][MF_OPTIONS + 2] = {};
-    int& n = known[model][dir][opt + 1];
+int warp_per_sm(int model, int fp64, int dir, int opt) {
+    static int known[2][2][2][MF_OPTIONS + 2] = {};
+    int& n = known[model][fp64][dir][opt + 1];
     if (!n) {
-        const WarpKernel k = warp_kernel(model, dir, opt);
+        const WarpKernel k = warp_kernel(model, fp64, dir, opt);
         int v = 0;
         const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k.fn, 128, k.smem);
         n = e != cudaSuccess || v < 1 ? 1 : v;
@@ -128,55 +141,18 @@ int warp_per_sm(int model, int dir, int opt) {
 
 // Persistent launch: as many warps as fit on the device (never more than
 // there are tiles), each walking every W-th tile.
-int launch_warp(int model, int dir, int opt, const MixedArgs& a, int sms, cudaStream_t st) {
-    const WarpKernel k = warp_kernel(model, dir, opt);
-    const int warps = std::max(1, std::min(a.ntiles, warp_per_sm(model, dir, opt) * sms * 4));
+int launch_warp(int model, int fp64, int dir, int opt, const MixedArgs& a, int sms, cudaStream_t st) {
+    const WarpKernel k = warp_kernel(model, fp64, dir, opt);
+    const int warps = std::max(1, std::min(a.ntiles, warp_per_sm(model, fp64, dir, opt) * sms * 4));
     k.fn<<<(warps + 3) / 4, 128, k.smem, st>>>(a);
     cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return cfd_fail(CFD_ERR_CUDA, "mixed sweep launch: %s", cudaGetErrorString(e));
-    return CFD_OK;
-}
-
-// The fast FP64 form's sweeps (cfd_fast64.cuh), launched like the mixed
-// warp forms: x by warp segments, y by marching strips.
-template <int MODEL>
-int march64_per_sm() {
-    static int per_sm = 0;
-    if (!per_sm) {
-        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &per_sm, fast::fast_march_kernel<MODEL>, 128, fast::march64_smem_bytes<MODEL>());
-        if (e != cudaSuccess || per_sm < 1) per_sm = 1;
-    }
-    return per_sm;
-}
-
-template <int MODEL>
-int segment64_per_sm() {
-    static int per_sm = 0;
-    if (!per_sm) {
-        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
-            &per_sm, fast::fast_segment_x_kernel<MODEL>, 128, fast::segment64_smem_bytes<MODEL>());
-        if (e != cudaSuccess || per_sm < 1) per_sm = 1;
-    }
-    return per_sm;
-}
-
-template <int MODEL>
-int launch_fast(int dir, const MixedArgs& a, int sms, cudaStream_t st) {
-    const int per_sm = dir == DIR_X ? segment64_per_sm<MODEL>() : march64_per_sm<MODEL>();
-    const int warps = std::max(1, std::min(a.ntiles, per_sm * sms * 4));
-    if (dir == DIR_X)
-        fast::fast_segment_x_kernel<MODEL><<<(warps + 3) / 4, 128, fast::segment64_smem_bytes<MODEL>(), st>>>(a);
-    else
-        fast::fast_march_kernel<MODEL><<<(warps + 3) / 4, 128, fast::march64_smem_bytes<MODEL>(), st>>>(a);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return cfd_fail(CFD_ERR_CUDA, "fast FP64 sweep launch: %s", cudaGetErrorString(e));
+    if (e != cudaSuccess) return cfd_fail(CFD_ERR_CUDA, "sweep launch: %s", cudaGetErrorString(e));
     return CFD_OK;
 }
 
 template <int MODEL>
 int launch_shape(int dir, int shape, int opt, const MixedArgs& a, int grid, cudaStream_t st) {
-    if (dir == DIR_X || shape == kMarchShape) return launch_warp(MODEL, dir, opt, a, grid, st);
+    if (dir == DIR_X || shape == kMarchShape) return launch_warp(MODEL, 0, dir, opt, a, grid, st);
     switch (shape) {
         case 0: return launch_t<MODEL, DIR_Y, 28, 8>(a, grid, st);
         case 1: return launch_t<MODEL, DIR_Y, 60, 4>(a, grid, st);
@@ -543,22 +519,16 @@ int build_tables(cfd_batch* b) {
             opt = kOptGeneral;
             for (const Member& m : b->members)
                 if (m.cfg.model == model && m.inst.fp64 == f64 && !m.final) {
-                    const int o = m.inst.flags & MF_OPTIONS;
+                    const int o = sweep_options(m.inst.flags);
                     opt = grids.empty() || o == opt ? o : kOptGeneral;
                     grids.emplace_back(m.cfg.nx, m.cfg.ny);
                 }
             if (grids.empty()) continue;
-            const int seg_sm =
-                f64 ? (model == CFD_MODEL_EULER ? segment64_per_sm<MODEL_EULER>()
-                                                : segment64_per_sm<MODEL_ALLAIRE>())
-                    : warp_per_sm(model, DIR_X, opt);
+            const int seg_sm = warp_per_sm(model, f64, DIR_X, opt);
             shape_x[model][f64].na = seg_rows(grids, (long long)seg_sm * b->sms * 4);
             b->seg_used[model][f64] = shape_x[model][f64].na;
             if (shp != kMarchShape) continue;
-            const int per_sm =
-                f64 ? (model == CFD_MODEL_EULER ? march64_per_sm<MODEL_EULER>()
-                                                : march64_per_sm<MODEL_ALLAIRE>())
-                    : warp_per_sm(model, DIR_Y, opt);
+            const int per_sm = warp_per_sm(model, f64, DIR_Y, opt);
             shape_y[model][f64].ts = b->march_fixed[model]
                                          ? b->march_fixed[model]
                                          : march_rows(grids, (long long)per_sm * b->sms * 4);
@@ -670,8 +640,7 @@ int enqueue_tick(cfd_batch* b, std::vector<Timed>* timing) {
             int grid = b->sms;
             int r;
             if (g.fp64)
-                r = g.model == CFD_MODEL_EULER ? launch_fast<MODEL_EULER>(dir, a, grid, b->stream)
-                                               : launch_fast<MODEL_ALLAIRE>(dir, a, grid, b->stream);
+                r = launch_warp(g.model, 1, dir, g.opt, a, grid, b->stream);
             else
                 r = g.model == CFD_MODEL_EULER
                         ? launch_shape<MODEL_EULER>(dir, g.shape, g.opt, a, grid, b->stream)

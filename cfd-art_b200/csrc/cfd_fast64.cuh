@@ -54,8 +54,15 @@ struct DPar {
     __device__ __forceinline__ int limiter() const { return flags & 3; }
     __device__ __forceinline__ bool pvrs() const { return (flags >> 2) & 1; }
     __device__ __forceinline__ bool godunov() const { return (flags >> 3) & 1; }
+    __device__ __forceinline__ bool stiff() const { return (flags >> 4) & 1; }
+    // p + p_inf and p + gamma p_inf (no addition for a gas)
+    __device__ __forceinline__ double plus_p1(double p) const { return stiff() ? p + p1 : p; }
+    __device__ __forceinline__ double plus_gp1(double p) const { return stiff() ? p + gp1 : p; }
 };
 
+// The parameters of an instance; OPT >= 0: the options its launch is compiled
+// for (cfd_march.cuh).
+template <int OPT>
 __device__ __forceinline__ DPar load_dpar(const Inst& I) {
     DPar P;
     P.g1 = I.eos.g1;
@@ -66,7 +73,8 @@ __device__ __forceinline__ DPar load_dpar(const Inst& I) {
     P.i2 = I.pd[1];
     P.c1 = I.pd[2];
     P.c2 = I.pd[3];
-    P.flags = I.flags;
+    P.flags = OPT >= 0 ? OPT : I.flags;
+    if (OPT >= 0 && !(OPT & mixed::MF_STIFF)) P.p1 = P.gp1 = P.c1 = P.c2 = 0.0;
     return P;
 }
 
@@ -80,16 +88,25 @@ __device__ __forceinline__ double rcp(double x) {
     return fma(y, fma(e, e, e), y);
 }
 
-// sqrt(a) = a / sqrt(a): the hardware approximation of 1/sqrt(a) refined by
-// one Householder step of order 3, y (1 + e/2 + 3 e^2/8) with e = 1 - a y^2;
-// 0 for a = 0 and NaN for a < 0, as sqrt gives.
-__device__ __forceinline__ double sqrt_f(double a) {
+// 1/sqrt(a): the hardware approximation refined by one Householder step of
+// order 3, y (1 + e/2 + 3 e^2/8) with e = 1 - a y^2.  The approximation is
+// taken of a + 1e-300, which is a for every a above 1e-284 and keeps y finite
+// for a = 0; NaN for a < 0.
+__device__ __forceinline__ double rsqrt_f(double a) {
     double y;
-    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a));
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(a + 1e-300));
     const double e = fma(-a * y, y, 1.0);
-    y = fma(y * fma(0.375, e, 0.5), e, y);
-    return a > 0.0 ? a * y : (a == 0.0 ? 0.0 : __longlong_as_double(0x7ff8000000000000LL));
+    return fma(y * fma(0.375, e, 0.5), e, y);
 }
+// sqrt(a), and sqrt(a / b) = a / sqrt(a b) without the division; 0 for a = 0.
+// (The products are not to be contracted into what follows, so that every
+// instantiation of a sweep gives the same bits.)
+__device__ __forceinline__ double sqrt_f(double a) { return __dmul_rn(a, rsqrt_f(a)); }
+__device__ __forceinline__ double sqrt_ratio(double a, double b) { return __dmul_rn(a, rsqrt_f(a * b)); }
+
+__device__ __forceinline__ int hi32(double x) { return __double2hiint(x); }
+constexpr unsigned kInfHi = 0x7ff00000u;   // high word of infinity
+constexpr unsigned kSnapHi = 0x3d720000u;  // just above 1e-12
 
 __device__ __forceinline__ double dmin(double a, double b) { return (b < a) ? b : a; }
 __device__ __forceinline__ double dmax(double a, double b) { return (a < b) ? b : a; }
@@ -110,7 +127,7 @@ template <int MODEL>
 __device__ __forceinline__ void mix_eps_kn(const DPar& P, double z, double& eps, double& kn) {
     const double omz = 1.0 - z;
     eps = fma(z, P.i1, omz * P.i2);
-    kn = fma(z, P.c1, omz * P.c2);
+    kn = P.stiff() ? fma(z, P.c1, omz * P.c2) : 0.0;
 }
 
 template <int MODEL>
@@ -122,7 +139,7 @@ __device__ __forceinline__ void c2p(const DPar& P, const double* U, Prim64<MODEL
         Q.W[0] = U[0];
         Q.W[1] = u;
         Q.W[2] = v;
-        Q.W[3] = fma(P.gm1, re, -P.gp1);
+        Q.W[3] = P.stiff() ? fma(P.gm1, re, -P.gp1) : P.gm1 * re;
     } else {
         Q.r = rcp(U[0] + U[1]);
         const double u = U[2] * Q.r, v = U[3] * Q.r;
@@ -143,7 +160,7 @@ __device__ __forceinline__ void c2p(const DPar& P, const double* U, Prim64<MODEL
 // (k + p (1/eps + 1)) for a mixture (A/headers/mixturemodel.hpp:34-40).
 template <int MODEL>
 __device__ __forceinline__ double rho_c2(const DPar& P, const double* W, double ie, double kn) {
-    if constexpr (MODEL == MODEL_EULER) return P.g1 * (W[3] + P.p1);
+    if constexpr (MODEL == MODEL_EULER) return P.g1 * P.plus_p1(W[3]);
     else return fma(kn + W[4], ie, W[4]);
 }
 
@@ -153,7 +170,7 @@ __device__ __forceinline__ double rho_c2(const DPar& P, const double* W, double 
 template <int MODEL>
 __device__ __forceinline__ bool phys(const DPar& P, double* W) {
     if constexpr (MODEL == MODEL_EULER) {
-        return W[0] > 0.0 && W[3] + P.gp1 >= 0.0;
+        return W[0] > 0.0 && P.plus_gp1(W[3]) >= 0.0;
     } else {
         if (fabs(W[0]) < 1e-12) W[0] = 0.0;
         if (fabs(W[1]) < 1e-12) W[1] = 0.0;
@@ -174,14 +191,18 @@ __device__ __forceinline__ double limit(int lim, double a, double b) {
             const double ab = a * b;
             return ab > 0.0 ? 2.0 * ab * rcp(a + b) : 0.0;
         }
-        case LIM_MC:
-            if (b >= 0.0 && a >= 0.0) return dmin(0.5 * (a + b), dmin(2.0 * a, 2.0 * b));
-            if (b <= 0.0 && a <= 0.0) return dmax(0.5 * (a + b), dmax(2.0 * a, 2.0 * b));
-            return 0.0;
+        case LIM_MC: {
+            // the smallest in size of (a + b)/2, 2 a, 2 b where the signs agree, else 0
+            const double x = 2.0 * (fabs(b) < fabs(a) ? b : a), m = 0.5 * (a + b);
+            return (hi32(a) ^ hi32(b)) >= 0 ? (fabs(m) < fabs(x) ? m : x) : 0.0;
+        }
         case LIM_UNLIMITED:
             return 0.5 * (a + b);
-        default:
-            return (b > 0.0) ? dmax(0.0, dmin(a, b)) : dmin(0.0, dmax(a, b));
+        default: {
+            // minmod: the smaller in size where the signs agree, else 0
+            const double x = fabs(b) < fabs(a) ? b : a;
+            return (hi32(a) ^ hi32(b)) >= 0 ? x : 0.0;
+        }
     }
 }
 
@@ -207,47 +228,81 @@ __device__ __forceinline__ void limit_all(int lim, const double* Wm, const doubl
     }
 }
 
+// The largest and the smallest high word of component q over four states.
+template <int NV>
+__device__ __forceinline__ void hi_range(int q, const double* a, const double* b, const double* c,
+                                         const double* d, unsigned& lo, unsigned& up) {
+    const unsigned x = hi32(a[q]), y = hi32(b[q]), z = hi32(c[q]), w = hi32(d[q]);
+    lo = min(min(x, y), min(z, w));
+    up = max(max(x, y), max(z, w));
+}
+
 // Evolved face states of a cell (E/headers/flux_solver_MUSCLhancock.hpp:195-201):
 // Wp/Wm = W +/- d/2 - (dt/(2 dx)) A(W) d with the primitive Jacobian of
 // E/headers/misc_euler.hpp:102-119 (A/headers/misc.hpp:189-205), zero entries
-// dropped; fl gets bit 0/1 for a physical slope-extrapolated high/low state
-// and bit 2/3 for a physical evolved high/low state.
+// dropped; okp / okm: the slope-extrapolated and the evolved high / low state
+// are physical.  Most cells pass on their high words alone: every density
+// normal and positive (Allaire: zero, or above the snapping threshold, as
+// z and 1 - z), every pressure positive or zero.  Those are sufficient, a
+// mixture's eps and eps k being >= 0, and leave nothing to snap; only other
+// cells are tested (and snapped) state by state.
 template <int MODEL>
 __device__ __forceinline__ void face_states(const DPar& P, const Prim64<MODEL>& Q, const double* d,
-                                            double s, double* Wp, double* Wm, unsigned& fl) {
+                                            double s, double* Wp, double* Wm, bool& okp, bool& okm) {
     constexpr int NV = ModelTraits<MODEL>::NV;
     const double* W = Q.W;
-    fl = 0;
-#pragma unroll
-    for (int q = 0; q < NV; ++q) Wp[q] = fma(0.5, d[q], W[q]);
-    if (phys<MODEL>(P, Wp)) fl |= 1u;
-#pragma unroll
-    for (int q = 0; q < NV; ++q) Wm[q] = fma(-0.5, d[q], W[q]);
-    if (phys<MODEL>(P, Wm)) fl |= 2u;
-    double X[NV];
+    double E[NV], D[NV], X[NV];
     const double rc2 = rho_c2<MODEL>(P, W, Q.ie, Q.kn);
     if constexpr (MODEL == MODEL_EULER) {
-        const double u = W[1];
-        X[0] = s * fma(u, d[0], W[0] * d[1]);
-        X[1] = s * fma(u, d[1], Q.r * d[3]);
-        X[2] = s * (u * d[2]);
-        X[3] = s * fma(rc2, d[1], u * d[3]);
+        const double su = s * W[1];
+        X[0] = fma(su, d[0], (s * W[0]) * d[1]);
+        X[1] = fma(su, d[1], (s * Q.r) * d[3]);
+        X[2] = su * d[2];
+        X[3] = fma(su, d[3], (s * rc2) * d[1]);
     } else {
-        const double u = W[2];
-        X[0] = s * fma(u, d[0], W[0] * d[2]);
-        X[1] = s * fma(u, d[1], W[1] * d[2]);
-        X[2] = s * fma(u, d[2], Q.r * d[4]);
-        X[3] = s * (u * d[3]);
-        X[4] = s * fma(rc2, d[2], u * d[4]);
-        X[5] = s * (u * d[5]);
+        const double su = s * W[2], sd = s * d[2];
+        X[0] = fma(su, d[0], W[0] * sd);
+        X[1] = fma(su, d[1], W[1] * sd);
+        X[2] = fma(su, d[2], (s * Q.r) * d[4]);
+        X[3] = su * d[3];
+        X[4] = fma(su, d[4], rc2 * sd);
+        X[5] = su * d[5];
     }
 #pragma unroll
     for (int q = 0; q < NV; ++q) {
-        Wp[q] = fma(0.5, d[q], W[q]) - X[q];
-        Wm[q] = fma(-0.5, d[q], W[q]) - X[q];
+        E[q] = fma(0.5, d[q], W[q]);
+        D[q] = fma(-0.5, d[q], W[q]);
+        Wp[q] = E[q] - X[q];
+        Wm[q] = D[q] - X[q];
     }
-    if (phys<MODEL>(P, Wp)) fl |= 4u;
-    if (phys<MODEL>(P, Wm)) fl |= 8u;
+    bool ok;
+    unsigned lo, up, lop, upp;
+    hi_range<NV>(0, E, D, Wp, Wm, lo, up);
+    if constexpr (MODEL == MODEL_EULER) {
+        hi_range<NV>(3, E, D, Wp, Wm, lop, upp);
+        ok = (lo >= 1u) & (max(up, upp) < kInfHi);
+    } else {
+        unsigned lo1, up1, lo5, up5;
+        hi_range<NV>(1, E, D, Wp, Wm, lo1, up1);
+        hi_range<NV>(4, E, D, Wp, Wm, lop, upp);
+        hi_range<NV>(5, E, D, Wp, Wm, lo5, up5);
+        // 1 - z of the four
+        const double o[4] = {1.0 - E[5], 1.0 - D[5], 1.0 - Wp[5], 1.0 - Wm[5]};
+        const unsigned loz = min(min((unsigned)hi32(o[0]), (unsigned)hi32(o[1])),
+                                 min((unsigned)hi32(o[2]), (unsigned)hi32(o[3])));
+        const unsigned upz = max(max((unsigned)hi32(o[0]), (unsigned)hi32(o[1])),
+                                 max((unsigned)hi32(o[2]), (unsigned)hi32(o[3])));
+        ok = (max(max(max(up, up1), max(upp, up5)), upz) < kInfHi) & ((lo >= kSnapHi) | (up == 0u)) &
+             ((lo1 >= kSnapHi) | (up1 == 0u)) & ((lo5 >= kSnapHi) | (up5 == 0u)) &
+             ((loz >= kSnapHi) | (upz == 0u)) & (max(lo, lo1) != 0u);
+    }
+    okp = okm = ok;
+    if (!ok) {
+        okp = phys<MODEL>(P, E);
+        okm = phys<MODEL>(P, D);
+        okp &= phys<MODEL>(P, Wp);
+        okm &= phys<MODEL>(P, Wm);
+    }
 }
 
 // Sound speed of a primitive state from its own reciprocals.
@@ -267,8 +322,8 @@ template <int MODEL>
 __device__ __forceinline__ void hllc(const DPar& P, const double* WL, const double* WR, double* F) {
     using T = ModelTraits<MODEL>;
     constexpr int NV = T::NV;
-    double rhoL, rhoR, uL, uR, pL, pR, rL, rR;
-    double eL = 1.0, eR = 1.0, ieL = 1.0, ieR = 1.0, knL = 0.0, knR = 0.0;  // Allaire: eps, 1/eps, eps k
+    double rhoL, rhoR, uL, uR, pL, pR, cL, cR;
+    double eL = 1.0, eR = 1.0, knL = 0.0, knR = 0.0, MLe = 0.0, MRe = 0.0;  // Allaire: eps, eps k, eps rho
     if constexpr (MODEL == MODEL_EULER) {
         rhoL = WL[0];
         rhoR = WR[0];
@@ -276,6 +331,8 @@ __device__ __forceinline__ void hllc(const DPar& P, const double* WL, const doub
         uR = WR[1];
         pL = WL[3];
         pR = WR[3];
+        cL = sqrt_ratio(P.g1 * P.plus_p1(pL), rhoL);
+        cR = sqrt_ratio(P.g1 * P.plus_p1(pR), rhoR);
     } else {
         rhoL = WL[0] + WL[1];
         rhoR = WR[0] + WR[1];
@@ -285,79 +342,61 @@ __device__ __forceinline__ void hllc(const DPar& P, const double* WL, const doub
         pR = WR[4];
         mix_eps_kn<MODEL>(P, WL[5], eL, knL);
         mix_eps_kn<MODEL>(P, WR[5], eR, knR);
-        ieL = rcp(eL);
-        ieR = rcp(eR);
+        // c^2 = (k + p (1/eps + 1))/rho = (eps k + p + p eps)/(eps rho)
+        MLe = eL * rhoL;
+        MRe = eR * rhoR;
+        cL = sqrt_ratio(fma(pL, eL, knL + pL), MLe);
+        cR = sqrt_ratio(fma(pR, eR, knR + pR), MRe);
     }
-    rL = rcp(rhoL);
-    rR = rcp(rhoR);
-    const double cL = sound<MODEL>(P, WL, rL, ieL, knL);
-    const double cR = sound<MODEL>(P, WR, rR, ieR, knR);
     double SL, SR;
     if (MODEL == MODEL_ALLAIRE && P.pvrs()) {
         const double ppv =
             dmax(0.0, fma(0.5, pL + pR, ((0.5 * (uL - uR)) * (0.5 * (rhoL + rhoR))) * (0.5 * (cL + cR))));
         // shock_speed_jump: sqrt(((p* + k) + ((p* + p)/2)/eps) / rho)
-        SL = ppv > pL ? uL - sqrt_f((fma(knL, ieL, ppv) + 0.5 * (ppv + pL) * ieL) * rL) : uL - cL;
-        SR = ppv > pR ? uR + sqrt_f((fma(knR, ieR, ppv) + 0.5 * (ppv + pR) * ieR) * rR) : uR + cR;
+        SL = uL - (ppv > pL ? sqrt_ratio(fma(ppv, eL, fma(0.5, ppv + pL, knL)), MLe) : cL);
+        SR = uR + (ppv > pR ? sqrt_ratio(fma(ppv, eR, fma(0.5, ppv + pR, knR)), MRe) : cR);
     } else {
         const double ua = 0.5 * (uL + uR), ca = 0.5 * (cL + cR);
         SL = dmin(ua - ca, uL - cL);
         SR = dmax(ua + ca, uR + cR);
     }
     const double mL = rhoL * (SL - uL), mR = rhoR * (SR - uR);
-    const double us = fma(mL, uL, pR - pL) - mR * uR;
-    const double u_star = us * rcp(mL - mR);
-    const bool left = !signbit(u_star);
+    // u* = num/den; its sign, and 1/(S - u*) = den/(S den - num), do not wait
+    // for the quotient
+    const double num = fma(-mR, uR, fma(mL, uL, pR - pL)), den = mL - mR;
+    const bool left = (hi32(num) ^ hi32(den)) >= 0;
     // per-element selects (a pointer to either side would go through local memory)
     const double rho = left ? rhoL : rhoR, u = left ? uL : uR, p = left ? pL : pR;
+    const double v = left ? WL[T::IT] : WR[T::IT];
     const double Sk = left ? SL : SR, wave = left ? dmin(0.0, SL) : dmax(0.0, SR);
-    const double q = rcp(Sk - u_star);   // 1/(S - u*)
-    const double fac = (Sk - u) * q;     // (S - u)/(S - u*)
-    double U[NV];
+    const double q = den * rcp(fma(Sk, den, -num));  // 1/(S - u*)
+    const double u_star = num * rcp(den);
+    const double fac = (Sk - u) * q;    // (S - u)/(S - u*)
+    // The passive components' flux U u + w (fac U - U) is U A; the normal
+    // momentum's rho (u^2 + w (fac u* - u)) + p; the energy's star state
+    // fac (E + (u* - u)(rho u* + p/(S - u))) - E gives E A + p u
+    // + w (u* - u)(fac rho u* + p/(S - u*))
+    const double A = fma(wave, fac - 1.0, u);
+    double re;
     if constexpr (MODEL == MODEL_EULER) {
-        const double v = left ? WL[2] : WR[2];
-        U[0] = rho;
-        U[1] = rho * u;
-        U[2] = rho * v;
-        U[3] = fma(p + P.gp1, P.i1, (0.5 * rho) * fma(u, u, v * v));
+        re = P.plus_gp1(p) * P.i1;
     } else {
-        const double v = left ? WL[3] : WR[3];
         const double eps = left ? eL : eR, kn = left ? knL : knR;
-        U[0] = left ? WL[0] : WR[0];
-        U[1] = left ? WL[1] : WR[1];
-        U[2] = rho * u;
-        U[3] = rho * v;
-        U[4] = fma(p, eps, kn) + (0.5 * rho) * fma(u, u, v * v);  // (p + k) eps + rho |u|^2 / 2
-        U[5] = left ? WL[5] : WR[5];
+        re = fma(p, eps, kn);  // (p + k) eps
     }
-    // star state: fac U, momentum fac rho u*, energy
-    // fac (E + (u* - u)(rho u* + p/(S - u))) = fac (E + (u* - u) rho u*) + (u* - u) p / (S - u*)
-    const double du = u_star - u;
-    double Us[NV];
-#pragma unroll
-    for (int k = 0; k < NV; ++k) Us[k] = fac * U[k];
-    Us[T::IM] = fac * (rho * u_star);
-    Us[T::IE] = fma(fac, fma(du, rho * u_star, U[T::IE]), du * (p * q));
-    double Fp[NV];
+    const double E = fma(0.5 * rho, fma(u, u, v * v), re);
+    const double m = rho * A, fu = fac * u_star;
     if constexpr (MODEL == MODEL_EULER) {
-        Fp[0] = U[1];
-        Fp[1] = fma(U[1], u, p);
-        Fp[2] = U[2] * u;
-        Fp[3] = (U[3] + p) * u;
+        F[0] = m;
     } else {
-        Fp[0] = U[0] * u;
-        Fp[1] = U[1] * u;
-        Fp[2] = fma(U[2], u, p);
-        Fp[3] = U[3] * u;
-        Fp[4] = (U[4] + p) * u;
-        Fp[5] = 0.0;
-    }
-#pragma unroll
-    for (int k = 0; k < NV; ++k) F[k] = fma(wave, Us[k] - U[k], Fp[k]);
-    if constexpr (MODEL == MODEL_ALLAIRE) {
+        F[0] = (left ? WL[0] : WR[0]) * A;
+        F[1] = (left ? WL[1] : WR[1]) * A;
         F[5] = 0.0;
-        F[NV + 1] = U[5];
+        F[NV + 1] = left ? WL[5] : WR[5];
     }
+    F[T::IM] = fma(rho, fma(wave, fu - u, u * u), p);
+    F[T::IT] = m * v;
+    F[T::IE] = fma(wave * (u_star - u), fma(rho, fu, p * q), fma(E, A, p * u));
     F[NV] = u_star;
 }
 
@@ -388,6 +427,10 @@ __device__ __forceinline__ bool euler_physical(const double* N) {
 template <int MODEL>
 __device__ __forceinline__ void repair(double* N, const double* Uold) {
     if constexpr (MODEL == MODEL_ALLAIRE) {
+        // nothing to snap where the four sizes clear the threshold
+        const unsigned lo = min(min((unsigned)hi32(N[0]) & 0x7fffffffu, (unsigned)hi32(N[1]) & 0x7fffffffu),
+                                min((unsigned)hi32(N[5]) & 0x7fffffffu, (unsigned)hi32(N[5] - 1.0) & 0x7fffffffu));
+        if (lo >= kSnapHi) return;
         if (fabs(N[0]) < 1e-12) N[0] = 0.0;
         if (fabs(N[1]) < 1e-12) N[1] = 0.0;
         if (fabs(N[5]) < 1e-12) N[5] = 0.0;
@@ -542,13 +585,13 @@ __device__ __forceinline__ void stage_read(const char* stg, int s, double* U) {
 // the evolved high-face state of row k - 2 and the partly updated state of
 // row k - 2 (its low-face flux applied); the raw state of row k - 1 is read
 // again from its staging slot (Euler) or carried (Allaire).
-template <int MODEL>
+template <int MODEL, int OPT>
 __device__ __forceinline__ void march64_strip(const MixedArgs& A, const TileGeom& g) {
     using MT = ModelTraits<MODEL>;
     constexpr int NV = MT::NV;
     const int lane = threadIdx.x & 31;
     const Inst& I = A.insts[g.inst];
-    const DPar P = load_dpar(I);
+    const DPar P = load_dpar<OPT>(I);
     DevState* st = I.st;
     const double dt = st->dt;
     const double s_half = 0.5 * (dt / (I.fix_dy ? I.dy : I.dx));  // the reference: dx (quirk)
@@ -562,7 +605,7 @@ __device__ __forceinline__ void march64_strip(const MixedArgs& A, const TileGeom
     // the x sweep's output -> the current buffer
     const Planes64 pin = planes64<MODEL>(I, g.cur ^ 1), pout = planes64<MODEL>(I, g.cur);
     const long long pitch = I.pitch;
-    const bool wall_lo = (P.flags >> 7) & 1, wall_hi = (P.flags >> 8) & 1;
+    const bool wall_lo = (I.flags >> 7) & 1, wall_hi = (I.flags >> 8) & 1;
     const bool god = P.godunov();
     const int lim = P.limiter();
     const double z_min = I.z_min;
@@ -582,7 +625,7 @@ __device__ __forceinline__ void march64_strip(const MixedArgs& A, const TileGeom
 
     Prim64<MODEL> Q1, Q2;          // rows k-1, k-2
     double A2[NV], Pp[NV];         // partly updated row k-2, high face of row k-2
-    unsigned flp = 0;
+    bool okp = false;              // whether Pp may be used
     double usL = 0.0, zsL = 0.0;   // u*, z* at the low face of row k-2
     double z3 = 0.0;               // z of row k-3 (upwind z update)
     double rmu = 0.0, rmv = 0.0, rm1 = 0.0, rm2 = 0.0;
@@ -632,11 +675,11 @@ __device__ __forceinline__ void march64_strip(const MixedArgs& A, const TileGeom
 
         // slope and face states of row k-1
         double Pn[NV], Mn[NV];
-        unsigned fln = 0;
+        bool okn = false, okm = false;
         if (k >= r0 && !god) {
             double d[NV];
             limit_all<NV>(lim, Q2.W, Q1.W, Q0.W, d);
-            face_states<MODEL>(P, Q1, d, s_half, Pn, Mn, fln);
+            face_states<MODEL>(P, Q1, d, s_half, Pn, Mn, okn, okm);
         } else {
 #pragma unroll
             for (int q = 0; q < NV; ++q) Pn[q] = Mn[q] = Q1.W[q];
@@ -644,14 +687,16 @@ __device__ __forceinline__ void march64_strip(const MixedArgs& A, const TileGeom
 
         if (k >= r0 + 1) {
             // flux at the face between rows k-2 and k-1
-            double F[NV + 2], WL[NV], WR[NV];
-            const bool second = !god && (flp & 1u) && (fln & 2u) && (flp & 4u) && (fln & 8u);
+            double F[NV + 2];
+            const bool first = god || !(okp && okm);
+            if (god || __any_sync(0xffffffffu, first)) {  // rare in second order
 #pragma unroll
-            for (int q = 0; q < NV; ++q) {
-                WL[q] = second ? Pp[q] : Q2.W[q];
-                WR[q] = second ? Mn[q] : Q1.W[q];
+                for (int q = 0; q < NV; ++q) {
+                    Pp[q] = first ? Q2.W[q] : Pp[q];
+                    Mn[q] = first ? Q1.W[q] : Mn[q];
+                }
             }
-            hllc<MODEL>(P, WL, WR, F);
+            hllc<MODEL>(P, Pp, Mn, F);
 
             if (k >= r0 + 2) {  // row k-2 is complete
                 const int row = k - 2;
@@ -714,7 +759,7 @@ __device__ __forceinline__ void march64_strip(const MixedArgs& A, const TileGeom
             Pp[q] = Pn[q];
             if constexpr (!reread) H1c[q] = h[q];
         }
-        flp = fln;
+        okp = okn;
     }
 
     // this strip's wave speeds and masses into its slot, then the ticket
@@ -743,13 +788,13 @@ __device__ __forceinline__ void march64_strip(const MixedArgs& A, const TileGeom
 
 // Euler bounded to 128 registers for 4 CTAs per SM: its y sweep measured
 // faster than at the 3 CTAs of its unbounded register count; Allaire runs 2.
-template <int MODEL>
+template <int MODEL, int OPT>
 __global__ void __launch_bounds__(128, MODEL == MODEL_EULER ? 4 : 2) fast_march_kernel(MixedArgs A) {
     const int gw = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int nw = gridDim.x * (blockDim.x >> 5);
     for (int tile = gw; tile < A.ntiles; tile += nw) {
         const TileGeom g = mixed::tile_geom<DIR_Y, mixed::kMarchMaxRows, 32>(A, tile);
-        if (!g.skip) march64_strip<MODEL>(A, g);
+        if (!g.skip) march64_strip<MODEL, OPT>(A, g);
     }
 }
 
@@ -774,13 +819,13 @@ __host__ __device__ constexpr int segment64_smem_bytes() {
     return 4 * kSegSlots * stage_units<MODEL>() * 32 * 16;  // 4 warps per CTA
 }
 
-template <int MODEL>
+template <int MODEL, int OPT>
 __device__ __forceinline__ void segment64_tile(const MixedArgs& A, const TileGeom& g) {
     using MT = ModelTraits<MODEL>;
     constexpr int NV = MT::NV;
     const int lane = threadIdx.x & 31;
     const Inst& I = A.insts[g.inst];
-    const DPar P = load_dpar(I);
+    const DPar P = load_dpar<OPT>(I);
     const double dt = I.st->dt;
     const double s_half = 0.5 * (dt / I.dx);
     const double k_upd = dt / I.dx;
@@ -796,10 +841,10 @@ __device__ __forceinline__ void segment64_tile(const MixedArgs& A, const TileGeo
     bool neg = false;
     if (ga < 0) {
         src = -ga - 1;
-        neg = (P.flags >> 5) & 1;
+        neg = (I.flags >> 5) & 1;
     } else if (ga >= nx) {
         src = 2 * nx - 1 - ga;
-        neg = (P.flags >> 6) & 1;
+        neg = (I.flags >> 6) & 1;
     }
     src = min(max(src, 0), nx - 1);
     const bool writer = lane >= 2 && lane < 2 + mixed::kSegCells && ga < nx;
@@ -827,34 +872,35 @@ __device__ __forceinline__ void segment64_tile(const MixedArgs& A, const TileGeo
         c2p<MODEL>(P, h, Q);
         double Wl[NV], Wr[NV];
         shfl_up64<NV>(Q.W, Wl);
-        shfl_down64<NV>(Q.W, Wr);
+        if (!god || MODEL == MODEL_ALLAIRE) shfl_down64<NV>(Q.W, Wr);  // first order: Allaire's z only
 
         // slope and face states of this cell (used by lanes 1..30)
         double Pf[NV], Mf[NV];
-        unsigned fl = 0;
+        bool okp = false, okm = false;
         if (!god) {
             double d[NV];
             limit_all<NV>(lim, Wl, Q.W, Wr, d);
-            face_states<MODEL>(P, Q, d, s_half, Pf, Mf, fl);
-        } else {
-#pragma unroll
-            for (int q = 0; q < NV; ++q) Pf[q] = Mf[q] = Q.W[q];
+            face_states<MODEL>(P, Q, d, s_half, Pf, Mf, okp, okm);
         }
 
         // HLLC at this cell's low face (between the lane below and this one)
         double F[NV + 2];
         {
             double PL[NV];
-            shfl_up64<NV>(Pf, PL);
-            const unsigned flL = __shfl_up_sync(0xffffffffu, fl, 1);
-            const bool second = !god && (flL & 1u) && (fl & 2u) && (flL & 4u) && (fl & 8u);
-            double WL[NV], WR[NV];
-#pragma unroll
-            for (int q = 0; q < NV; ++q) {
-                WL[q] = second ? PL[q] : Wl[q];
-                WR[q] = second ? Mf[q] : Q.W[q];
+            unsigned okL = 0;  // bit l: lane l - 1's high-face state may be used
+            if (!god) {
+                shfl_up64<NV>(Pf, PL);
+                okL = __ballot_sync(0xffffffffu, okp) << 1;
             }
-            hllc<MODEL>(P, WL, WR, F);
+            const bool first = god || (!(((okL >> lane) & 1u) && okm) && lane >= 2);
+            if (god || __any_sync(0xffffffffu, first)) {  // rare in second order
+#pragma unroll
+                for (int q = 0; q < NV; ++q) {
+                    PL[q] = first ? Wl[q] : PL[q];
+                    Mf[q] = first ? Q.W[q] : Mf[q];
+                }
+            }
+            hllc<MODEL>(P, PL, Mf, F);
         }
         double FR[NV + 2];  // Euler's update needs only the NV fluxes, not u*
         shfl_down64<MODEL == MODEL_EULER ? NV : NV + 2>(F, FR);
@@ -872,16 +918,26 @@ __device__ __forceinline__ void segment64_tile(const MixedArgs& A, const TileGeo
     }
 }
 
-// At least 4 CTAs per SM: Allaire bounded to 128 registers measured 25 %
-// faster than at the 3 CTAs of its unbounded count; Euler (96 registers)
-// runs 5.
-template <int MODEL>
-__global__ void __launch_bounds__(128, 4) fast_segment_x_kernel(MixedArgs A) {
+// Euler 5 CTAs per SM (96 registers), Allaire 4 (128: 25 % faster than the 3
+// of its unbounded count when that was measured); 6 and 5 spill and measured
+// 5 and 11 % slower.
+//
+// Both sweeps wait on FP64 latency at 16-20 warps per SM, with the FP64 pipe
+// half busy: at 2048^2 Euler the x sweep runs 375 thread instructions a cell,
+// about 155 of them FP64, and the y sweep 393, against 533 and 520 before
+// minmod took seven instructions, the physicality tests were made on high
+// words, first-order faces were left to a vote, HLLC's star state was reduced
+// to one reciprocal that does not wait for u*, sound speeds took one
+// reciprocal root and the options were fixed at compile time: x 96.7 -> 74.5
+// us, y 108.4 -> 90.7 us a sweep.  Allaire at 2048x1024 (880 -> 580
+// instructions in x): x 90.6 -> 63.8 us, y 121.1 -> 87.6 us.
+template <int MODEL, int OPT>
+__global__ void __launch_bounds__(128, MODEL == MODEL_EULER ? 5 : 4) fast_segment_x_kernel(MixedArgs A) {
     const int gw = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int nw = gridDim.x * (blockDim.x >> 5);
     for (int tile = gw; tile < A.ntiles; tile += nw) {
         const TileGeom g = mixed::tile_geom<DIR_X, mixed::kSegCells, mixed::kSegRows>(A, tile);
-        if (!g.skip) segment64_tile<MODEL>(A, g);
+        if (!g.skip) segment64_tile<MODEL, OPT>(A, g);
     }
 }
 

@@ -142,15 +142,12 @@ __device__ __forceinline__ void mstage_read(const char* slot, float* h, float* l
     }
 }
 
-// The options of a member as the sweeps branch on them (Inst::flags without
-// the walls), and the sets of them that have their own instantiations: minmod
-// and van Leer slopes of a gas (Euler), minmod slopes with PVRS speeds of a
-// stiffened gas and minmod slopes of two gases (Allaire).
+// The options of a member as the sweeps branch on them: Inst::flags without
+// the walls, and without the limiter in first order.
 constexpr int MF_OPTIONS = 31;
 constexpr int kOptGeneral = -1;
-template <int MODEL> __host__ __device__ constexpr int common_options(int i) {
-    return MODEL == MODEL_EULER ? (i == 0 ? LIM_MINMOD : LIM_VANLEER)
-                                : (i == 0 ? (LIM_MINMOD | MF_PVRS | MF_STIFF) : LIM_MINMOD);
+__host__ __device__ constexpr int sweep_options(int flags) {
+    return flags & MF_GODUNOV ? flags & MF_OPTIONS & ~3 : flags & MF_OPTIONS;
 }
 
 // One strip: rows [r0, r1) of the columns [b_org, b_org + 32) of instance
@@ -268,14 +265,15 @@ __device__ __forceinline__ void march_strip(const MixedArgs& A, const TileGeom& 
         // HLLC at the face between rows k-2 and k-1
         float Fh[NV + 2];
         if (steady || k >= r0 + 1) {
-            float WL[NV], WR[NV];
-            const bool second = okp && okm;  // else first order
+            const bool first = god || !(okp && okm);
+            if (god || __any_sync(0xffffffffu, first)) {  // rare in second order
 #pragma unroll
-            for (int q = 0; q < NV; ++q) {
-                WL[q] = second ? Pp[q] : W2[q];
-                WR[q] = second ? Mn[q] : W1[q];
+                for (int q = 0; q < NV; ++q) {
+                    Pp[q] = first ? W2[q] : Pp[q];
+                    Mn[q] = first ? W1[q] : Mn[q];
+                }
             }
-            hllc_prim<MODEL>(P, WL, WR, Fh);
+            hllc_prim<MODEL>(P, Pp, Mn, Fh);
         }
 
         // compensated update of row k-2
@@ -309,17 +307,17 @@ __device__ __forceinline__ void march_strip(const MixedArgs& A, const TileGeom& 
             c2p_mixed<MODEL>(I, P, hh, ll, Wn);
             if constexpr (MODEL == MODEL_EULER) {
                 // density / energy restore as in the plain form (rare)
-                if (!(hh[0] > 1e-12f) || !(Wn[3] + P.gp1 > 0.0f)) {
+                if (!(hh[0] > 1e-12f) || !(P.plus_gp1(Wn[3]) > 0.0f)) {
                     float oh[NV], ol[NV], Wo[NV];  // the cell before the update
                     load_cell<MODEL>(qin(), off, oh, ol);
                     c2p_mixed<MODEL>(I, P, oh, ol, Wo);  // stored (unrotated) frame
                     float rho = hh[0] > 1e-12f ? hh[0] : oh[0];
                     float u = Wn[1], v = Wn[2];
-                    float p = (Wn[3] + P.gp1 > 0.0f) ? Wn[3] : Wo[3];
+                    float p = (P.plus_gp1(Wn[3]) > 0.0f) ? Wn[3] : Wo[3];
                     hh[0] = rho; ll[0] = 0.f;
                     hh[1] = rho * u; ll[1] = 0.f;
                     hh[2] = rho * v; ll[2] = 0.f;
-                    hh[3] = (p + P.gp1) * P.i1 + 0.5f * rho * (u * u + v * v); ll[3] = 0.f;
+                    hh[3] = P.plus_gp1(p) * P.i1 + 0.5f * rho * (u * u + v * v); ll[3] = 0.f;
                     Wn[0] = rho;
                     Wn[3] = p;
                 }
@@ -496,7 +494,7 @@ __device__ __forceinline__ void segment_tile(const MixedArgs& A, const TileGeom&
         float W[NV], Wl[NV], Wr[NV];
         c2p_mixed<MODEL>(I, P, h, l, W);
         shfl_up_n<NV>(W, Wl);
-        shfl_down_n<NV>(W, Wr);
+        if (!god || MODEL == MODEL_ALLAIRE) shfl_down_n<NV>(W, Wr);  // first order: Allaire's z only
 
         // slopes and evolved face states of this cell (used by lanes 1..30)
         float Pf[NV], Mf[NV];
@@ -505,25 +503,28 @@ __device__ __forceinline__ void segment_tile(const MixedArgs& A, const TileGeom&
             float d[NV];
             limit_all<NV>(lim, Wl, W, Wr, d);
             face_states<MODEL>(P, W, d, s_half, Pf, Mf, okp, okm);
-        } else {
-#pragma unroll
-            for (int q = 0; q < NV; ++q) Pf[q] = Mf[q] = W[q];
         }
 
         // HLLC at this cell's low face (between the lane below and this one)
         float PL[NV];
-        shfl_up_n<NV>(Pf, PL);
-        const unsigned okL = __ballot_sync(0xffffffffu, okp) << 1;  // bit l: lane l - 1
+        unsigned okL = 0;  // bit l: lane l - 1's high-face state may be used
+        if (!god) {
+            shfl_up_n<NV>(Pf, PL);
+            okL = __ballot_sync(0xffffffffu, okp) << 1;
+        }
         float F[NV + 2];
         {
-            float WL[NV], WR[NV];
-            const bool second = ((okL >> lane) & 1u) && okm;  // else first order
+            const bool first = god || (!(((okL >> lane) & 1u) && okm) && lane >= 2);
+            // rare in second order (the vote measured 2 % faster than
+            // selecting for Allaire, 3 % slower for Euler)
+            if (MODEL == MODEL_EULER || god || __any_sync(0xffffffffu, first)) {
 #pragma unroll
-            for (int q = 0; q < NV; ++q) {
-                WL[q] = second ? PL[q] : Wl[q];
-                WR[q] = second ? Mf[q] : W[q];
+                for (int q = 0; q < NV; ++q) {
+                    PL[q] = first ? Wl[q] : PL[q];
+                    Mf[q] = first ? W[q] : Mf[q];
+                }
             }
-            hllc_prim<MODEL>(P, WL, WR, F);
+            hllc_prim<MODEL>(P, PL, Mf, F);
         }
         float FR[NV + 2];  // Euler's update needs only the NV fluxes, not u*
         shfl_down_n<MODEL == MODEL_EULER ? NV : NV + 2>(F, FR);
@@ -549,7 +550,7 @@ __device__ __forceinline__ void segment_tile(const MixedArgs& A, const TileGeom&
             bool restore = writer && !euler_sure(h);
             if (restore) {
                 c2p_mixed<MODEL>(I, P, h, l, Wn);
-                restore = !(h[0] > 1e-12f) || !(Wn[3] + P.gp1 > 0.0f);
+                restore = !(h[0] > 1e-12f) || !(P.plus_gp1(Wn[3]) > 0.0f);
             }
             if (restore) {
                 float oh[NV], ol[NV], Wo[NV];  // the cell before the update
@@ -557,11 +558,11 @@ __device__ __forceinline__ void segment_tile(const MixedArgs& A, const TileGeom&
                 c2p_mixed<MODEL>(I, P, oh, ol, Wo);
                 float rho = h[0] > 1e-12f ? h[0] : oh[0];
                 float u = Wn[1], v = Wn[2];
-                float p = (Wn[3] + P.gp1 > 0.0f) ? Wn[3] : Wo[3];
+                float p = (P.plus_gp1(Wn[3]) > 0.0f) ? Wn[3] : Wo[3];
                 h[0] = rho; l[0] = 0.f;
                 h[1] = rho * u; l[1] = 0.f;
                 h[2] = rho * v; l[2] = 0.f;
-                h[3] = (p + P.gp1) * P.i1 + 0.5f * rho * (u * u + v * v); l[3] = 0.f;
+                h[3] = P.plus_gp1(p) * P.i1 + 0.5f * rho * (u * u + v * v); l[3] = 0.f;
             }
         }
         if (writer) store_cell<MODEL>(qout, off_out, h, l);

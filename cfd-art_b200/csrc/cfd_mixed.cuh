@@ -89,6 +89,9 @@ struct MPar {
     __device__ __forceinline__ bool pvrs() const { return (flags >> 2) & 1; }
     __device__ __forceinline__ bool godunov() const { return (flags >> 3) & 1; }
     __device__ __forceinline__ bool stiff() const { return (flags >> 4) & 1; }
+    // p + p_inf and p + gamma p_inf (no addition for a gas)
+    __device__ __forceinline__ float plus_p1(float p) const { return stiff() ? p + p1 : p; }
+    __device__ __forceinline__ float plus_gp1(float p) const { return stiff() ? p + gp1 : p; }
 };
 enum { MF_PVRS = 4, MF_GODUNOV = 8, MF_STIFF = 16, MF_BC = 32 };  // MF_BC << k: wall on side k (L, R, B, T)
 
@@ -129,7 +132,12 @@ __device__ __forceinline__ float frcp(float x) { return 1.0f / x; }
 // a wave speed or a product of them, is many orders of magnitude smaller).
 // Measured 3-4 % faster on the sweeps, the same results on every test case.
 __device__ __forceinline__ float fdiv(float a, float b) { return __fdividef(a, b); }
-__device__ __forceinline__ float fsqrt(float x) { return sqrtf(x); }
+// sqrt(a / b) for b > 0 as a / sqrt(a b), with a at least 1e-30 (a root of
+// 1e-15 where it is 0 or negative): two instructions beside the hardware's.
+__device__ __forceinline__ float sqrt_ratio(float a, float b) {
+    const float x = fmaxf(a, 1e-30f);
+    return __fmul_rn(x, rsqrtf(x * b));
+}
 // One instruction each (the comparison forms of the reference's std::min and
 // std::max take two); a NaN operand gives the other one.
 __device__ __forceinline__ float fminf_s(float a, float b) { return fminf(a, b); }
@@ -195,7 +203,7 @@ __device__ __forceinline__ void pairs(Fn fn) {
 __device__ __forceinline__ void mix_f(const MPar& P, float z, float& eps, float& kn) {
     const float omz = 1.0f - z;
     eps = z * P.i1 + omz * P.i2;
-    kn = z * P.c1 + omz * P.c2;
+    kn = P.stiff() ? z * P.c1 + omz * P.c2 : 0.0f;
 }
 
 // Primitive state (rho-split for Allaire: W = rho1 z, rho2 (1-z), u, v, p, z).
@@ -267,14 +275,14 @@ __device__ __forceinline__ void c2p_mixed(const Inst& I, const MPar& P, const fl
 // fluxes on unlimited slopes at a contact).
 template <int MODEL> __device__ __forceinline__ bool phys_prim(const MPar& P, const float* W) {
     if constexpr (MODEL == MODEL_EULER) {
-        return W[0] > 0.0f && W[3] + P.gp1 >= 0.0f;
+        return W[0] > 0.0f && P.plus_gp1(W[3]) >= 0.0f;
     } else {
         // p + k >= 0  <=>  p eps + kn >= 0 (eps > 0 for 0 <= z <= 1)
         float omz = 1.0f - W[5];
         float eps = W[5] * P.i1 + omz * P.i2, kn = W[5] * P.c1 + omz * P.c2;
         // all six tests evaluated (no short-circuit branches): 2 % faster
         return (W[0] >= 0.0f) & (W[1] >= 0.0f) & (W[0] + W[1] > 0.0f) & (W[5] >= 0.0f) &
-               (W[5] <= 1.0f) & (W[4] * eps + kn >= 0.0f);
+               (W[5] <= 1.0f) & (fmaf(W[4], eps, kn) >= 0.0f);
     }
 }
 
@@ -333,13 +341,13 @@ __device__ __forceinline__ void limit_all(int lim, const float* Wm, const float*
 // Sound speed of a primitive state.
 template <int MODEL> __device__ __forceinline__ float sound_f(const MPar& P, const float* W) {
     if constexpr (MODEL == MODEL_EULER) {
-        return fsqrt(fmaxf_s(0.0f, fdiv(P.g1 * (W[3] + P.p1), W[0])));
+        return sqrt_ratio(P.g1 * P.plus_p1(W[3]), W[0]);
     } else {
         // c^2 = (k + p (1/eps + 1)) / rho = (kn + p (1 + eps)) / (eps rho)
         float omz = 1.0f - W[5];
         float eps = W[5] * P.i1 + omz * P.i2, kn = W[5] * P.c1 + omz * P.c2;
         float rho = W[0] + W[1];
-        return fsqrt(fmaxf_s(0.0f, fdiv(kn + W[4] * (1.0f + eps), eps * rho)));
+        return sqrt_ratio(fmaf(W[4], 1.0f + eps, kn), eps * rho);
     }
 }
 
@@ -350,7 +358,7 @@ __device__ __forceinline__ void jac_f(const MPar& P, const float* W, const float
                                       float* X) {
     if constexpr (MODEL == MODEL_EULER) {
         const float rho = W[0], u = W[1];
-        const float rc2 = fmaxf(0.0f, P.g1 * (W[3] + P.p1));
+        const float rc2 = fmaxf(0.0f, P.g1 * P.plus_p1(W[3]));
         X[0] = s * (u * d[0] + rho * d[1]);
         X[1] = s * (u * d[1] + frcp(rho) * d[3]);
         X[2] = s * (u * d[2]);
@@ -359,7 +367,7 @@ __device__ __forceinline__ void jac_f(const MPar& P, const float* W, const float
         const float rho = W[0] + W[1], u = W[2];
         float eps, kn;
         mix_f(P, W[5], eps, kn);
-        const float rc2 = fmaxf(0.0f, fdiv(kn + W[4] * (1.0f + eps), eps));
+        const float rc2 = fmaxf(0.0f, fdiv(fmaf(W[4], 1.0f + eps, kn), eps));
         X[0] = s * (u * d[0] + W[0] * d[2]);
         X[1] = s * (u * d[1] + W[1] * d[2]);
         X[2] = s * (u * d[2] + frcp(rho) * d[4]);
@@ -395,7 +403,7 @@ __device__ __forceinline__ void face_states(const MPar& P, const float* W, const
         return fmin_n(fmin_n(E[q], D[q]), fmin_n(Wp[q], Wm[q]));
     };
     if constexpr (MODEL == MODEL_EULER) {
-        all = (least(0) > 0.0f) & (least(3) + P.gp1 >= 0.0f);
+        all = (least(0) > 0.0f) & (P.plus_gp1(least(3)) >= 0.0f);
     } else {
         const float zm = fmax_n(fmax_n(E[5], D[5]), fmax_n(Wp[5], Wm[5]));
         const float r1 = least(0), r2 = least(1);
@@ -409,6 +417,11 @@ __device__ __forceinline__ void face_states(const MPar& P, const float* W, const
     }
 }
 
+// (Multiply-adds beside terms that vanish for a gas are written as fmaf: where
+// a launch's options make such a term a constant 0, the compiler would
+// otherwise contract the rest differently, and a member's bits would depend on
+// its company.)
+//
 // HLLC flux from primitive face states (same wave-speed estimates and star
 // states as hllc_flux in cfd_physics.cuh), F[NV] = u*, F[NV+1] = z* (Allaire).
 // With the star factor f = (S - u)/(S - u*), the passive components' flux
@@ -421,29 +434,29 @@ __device__ __forceinline__ void hllc_prim(const MPar& P, const float* WL, const 
     using T = ModelTraits<MODEL>;
     constexpr int NV = T::NV;
     float rL, rR, uL, uR, pL, pR, cL, cR, epsL = 1.f, knL = 0.f, epsR = 1.f, knR = 0.f;
-    float qL = 0.f, qR = 0.f;  // 1/(eps rho)
+    float qL = 1.f, qR = 1.f;  // eps rho
     if constexpr (MODEL == MODEL_EULER) {
         rL = WL[0]; uL = WL[1]; pL = WL[3];
         rR = WR[0]; uR = WR[1]; pR = WR[3];
-        cL = fsqrt(fmaxf(0.0f, fdiv(P.g1 * (pL + P.p1), rL)));
-        cR = fsqrt(fmaxf(0.0f, fdiv(P.g1 * (pR + P.p1), rR)));
+        cL = sqrt_ratio(P.g1 * P.plus_p1(pL), rL);
+        cR = sqrt_ratio(P.g1 * P.plus_p1(pR), rR);
     } else {
         rL = WL[0] + WL[1]; uL = WL[2]; pL = WL[4];
         rR = WR[0] + WR[1]; uR = WR[2]; pR = WR[4];
         mix_f(P, WL[5], epsL, knL);
         mix_f(P, WR[5], epsR, knR);
-        qL = frcp(epsL * rL);
-        qR = frcp(epsR * rR);
-        cL = fsqrt(fmaxf(0.0f, (knL + pL * (1.0f + epsL)) * qL));
-        cR = fsqrt(fmaxf(0.0f, (knR + pR * (1.0f + epsR)) * qR));
+        qL = epsL * rL;
+        qR = epsR * rR;
+        cL = sqrt_ratio(fmaf(pL, 1.0f + epsL, knL), qL);
+        cR = sqrt_ratio(fmaf(pR, 1.0f + epsR, knR), qR);
     }
     float SL, SR;
     if (MODEL == MODEL_ALLAIRE && P.pvrs()) {
         const float ra = 0.5f * (rL + rR), ca = 0.5f * (cL + cR);
         const float ppv = fmaxf(0.0f, 0.5f * (pL + pR) + 0.5f * (uL - uR) * ra * ca);
         // shock_speed_jump: sqrt(((p* + k) + ((p* + p)/2)/eps) / rho)
-        SL = uL - (ppv > pL ? fsqrt(fmaxf(0.0f, (knL + ppv * epsL + 0.5f * (ppv + pL)) * qL)) : cL);
-        SR = uR + (ppv > pR ? fsqrt(fmaxf(0.0f, (knR + ppv * epsR + 0.5f * (ppv + pR)) * qR)) : cR);
+        SL = uL - (ppv > pL ? sqrt_ratio(fmaf(ppv, epsL, fmaf(0.5f, ppv + pL, knL)), qL) : cL);
+        SR = uR + (ppv > pR ? sqrt_ratio(fmaf(ppv, epsR, fmaf(0.5f, ppv + pR, knR)), qR) : cR);
     } else {
         const float ua = 0.5f * (uL + uR), ca = 0.5f * (cL + cR);
         SL = fminf(ua - ca, uL - cL);
@@ -463,12 +476,12 @@ __device__ __forceinline__ void hllc_prim(const MPar& P, const float* WL, const 
     const float A = u + wave * (fac - 1.0f);
     float re;  // rho e
     if constexpr (MODEL == MODEL_EULER) {
-        re = (p + P.gp1) * P.i1;
+        re = P.plus_gp1(p) * P.i1;
     } else {
         const float eps = left ? epsL : epsR, kn = left ? knL : knR;
-        re = p * eps + kn;
+        re = fmaf(p, eps, kn);
     }
-    const float E = re + 0.5f * rho * (u * u + v * v);
+    const float E = fmaf(0.5f * rho, fmaf(u, u, v * v), re);
     const float m = rho * A;
     if constexpr (MODEL == MODEL_EULER) {
         F[0] = m;
@@ -862,7 +875,7 @@ __device__ __forceinline__ void mixed_tile(const MixedArgs& A, const TileGeom& g
             c2p_mixed<MODEL>(I, P, hh, ll, Wn);
             if constexpr (MODEL == MODEL_EULER) {
                 // density / energy restore as in the plain form (rare)
-                if (!(hh[0] > 1e-12f) || !(Wn[3] + P.gp1 > 0.0f)) {
+                if (!(hh[0] > 1e-12f) || !(P.plus_gp1(Wn[3]) > 0.0f)) {
                     float oh[NV], ol[NV], Wo[NV];  // the cell before the update
                     sH.get(s, oh);
                     sL.get(s, ol);
@@ -874,11 +887,11 @@ __device__ __forceinline__ void mixed_tile(const MixedArgs& A, const TileGeom& g
                     c2p_mixed<MODEL>(I, P, oh, ol, Wo);
                     float rho = hh[0] > 1e-12f ? hh[0] : oh[0];
                     float u = Wn[1], v = Wn[2];
-                    float p = (Wn[3] + P.gp1 > 0.0f) ? Wn[3] : Wo[3];
+                    float p = (P.plus_gp1(Wn[3]) > 0.0f) ? Wn[3] : Wo[3];
                     hh[0] = rho; ll[0] = 0.f;
                     hh[1] = rho * u; ll[1] = 0.f;
                     hh[2] = rho * v; ll[2] = 0.f;
-                    hh[3] = (p + P.gp1) * P.i1 + 0.5f * rho * (u * u + v * v); ll[3] = 0.f;
+                    hh[3] = P.plus_gp1(p) * P.i1 + 0.5f * rho * (u * u + v * v); ll[3] = 0.f;
                     Wn[0] = rho;
                     Wn[3] = p;
                 }
