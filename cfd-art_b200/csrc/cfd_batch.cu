@@ -143,7 +143,7 @@ int warp_per_sm(int model, int fp64, int dir, int opt) {
 // there are tiles), each walking every W-th tile.
 int launch_warp(int model, int fp64, int dir, int opt, const MixedArgs& a, int sms, cudaStream_t st) {
     const WarpKernel k = warp_kernel(model, fp64, dir, opt);
-    const int warps = std::max(1, std::min(a.ntiles, warp_per_sm(model, fp64, dir, opt) * sms * 4));
+    const int warps = std::max(1, std::min(a.ntiles * a.split, warp_per_sm(model, fp64, dir, opt) * sms * 4));
     k.fn<<<(warps + 3) / 4, 128, k.smem, st>>>(a);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cfd_fail(CFD_ERR_CUDA, "sweep launch: %s", cudaGetErrorString(e));
@@ -432,7 +432,13 @@ struct Member {
     void* mem = nullptr;  // one allocation: buffers, state, partials
     size_t bytes = 0;
     int max_steps;
+    int nslots;           // reduction slots of its allocation
 };
+
+// Division of tiles among warps (Group::split): while the launch's warps stay
+// at kSplitWarps per SM (two per scheduler) and a part of a strip keeps
+// kMinPartRows rows beside its 4 halo rows.
+constexpr int kSplitWarps = 16, kMinPartRows = 2;
 
 }  // namespace
 
@@ -451,8 +457,10 @@ struct cfd_batch {
         int model, fp64, dir, shape, ntiles, offset;
         int rows;  // marching strips: cells along the sweep per strip
         int opt;   // the options all its members share, or kOptGeneral
+        int split; // warp sweeps: parts (warps) per tile
     };
     std::vector<Group> groups;
+    bool close = false;  // some members' steps are closed by close_steps
     bool dirty = true;
     // [model][dir]; y sweeps march by default (measured fastest on B200 for
     // both models, and the strips adapt to the members)
@@ -501,6 +509,7 @@ int build_tables(cfd_batch* b) {
     if (int r = wait_uploads(b)) return r;
     if (!b->dirty) return CFD_OK;
     b->groups.clear();
+    b->close = false;
     // the x segments' row count and the y shape of each (model, form), with
     // the strip length of a marching sweep; the fast FP64 form always
     // marches in y
@@ -561,6 +570,7 @@ int build_tables(cfd_batch* b) {
                 g.shape = f64 ? (dir == DIR_X ? 0 : kMarchShape) : b->shape[model][dir];
                 g.offset = (int)all.size();
                 g.opt = opts[model][f64];
+                double slots = 0.0;  // the largest share of a member's reduction slots in use
                 const Shape sh = dir == DIR_X ? shape_x[model][f64] : shape_y[model][f64];
                 g.rows = dir == DIR_X ? sh.na : sh.ts;
                 for (int idx : order) {
@@ -571,6 +581,7 @@ int build_tables(cfd_batch* b) {
                     const int wid = dir == DIR_X ? m.cfg.ny : m.cfg.nx;
                     const int along = (len + sh.ts - 1) / sh.ts;
                     const int nt = dir == DIR_X ? insts[idx].tiles_x : insts[idx].tiles_y;
+                    slots = std::max(slots, (double)nt / m.nslots);
                     for (int t = 0; t < nt; ++t) {
                         TileEnt e;
                         e.inst = idx;
@@ -585,6 +596,20 @@ int build_tables(cfd_batch* b) {
                     }
                 }
                 g.ntiles = (int)all.size() - g.offset;
+                g.split = 1;
+                if (dir == DIR_X || g.shape == kMarchShape)
+                    while (g.ntiles * g.split * 2 <= kSplitWarps * b->sms &&
+                           g.rows >= g.split * 2 * (dir == DIR_X ? 1 : kMinPartRows) &&
+                           (dir == DIR_X || slots * g.split * 2 <= 1.0))
+                        g.split *= 2;
+                if (dir == DIR_Y && g.shape == kMarchShape)
+                    for (int idx : order) {
+                        const Member& m = b->members[idx];
+                        if (m.cfg.model != model || m.inst.fp64 != f64 || m.final) continue;
+                        insts[idx].slots = insts[idx].tiles_y * g.split;
+                        insts[idx].closed = insts[idx].slots > kTicketSlots;
+                        b->close |= insts[idx].closed != 0;
+                    }
                 if (g.ntiles) b->groups.push_back(g);
             }
     if ((int)insts.size() > b->d_insts_cap) {
@@ -621,7 +646,28 @@ struct Timed {
     cudaEvent_t e0, e1;
 };
 
+// close_steps behind the y sweep just launched, as its programmatic
+// dependent: scheduled while that sweep ends, it waits for its completion (and
+// that sweep for all before it, being an ordinary launch).
+int launch_close(const Inst* insts, int members, cudaStream_t st) {
+    cudaLaunchConfig_t c = {};
+    c.gridDim = dim3(members);
+    c.blockDim = dim3(kCloseThreads);
+    c.stream = st;
+    cudaLaunchAttribute a = {};
+    a.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    a.val.programmaticStreamSerializationAllowed = 1;
+    c.attrs = &a;
+    c.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&c, close_steps, insts);
+    if (e != cudaSuccess) return cfd_fail(CFD_ERR_CUDA, "closing steps: %s", cudaGetErrorString(e));
+    return CFD_OK;
+}
+
 int enqueue_tick(cfd_batch* b, std::vector<Timed>* timing) {
+    int last_y = -1;  // the last y launch, behind which close_steps follows
+    for (int gi = 0; gi < (int)b->groups.size(); ++gi)
+        if (b->groups[gi].dir == DIR_Y) last_y = gi;
     for (int dir = 0; dir < 2; ++dir)
         for (int gi = 0; gi < (int)b->groups.size(); ++gi) {
             const auto& g = b->groups[gi];
@@ -631,6 +677,7 @@ int enqueue_tick(cfd_batch* b, std::vector<Timed>* timing) {
             a.tiles = b->d_tiles + g.offset;
             a.ntiles = g.ntiles;
             a.rows = g.rows;
+            a.split = g.split;
             cudaEvent_t e0 = nullptr, e1 = nullptr;
             if (timing) {
                 cudaEventCreate(&e0);
@@ -645,6 +692,9 @@ int enqueue_tick(cfd_batch* b, std::vector<Timed>* timing) {
                 r = g.model == CFD_MODEL_EULER
                         ? launch_shape<MODEL_EULER>(dir, g.shape, g.opt, a, grid, b->stream)
                         : launch_shape<MODEL_ALLAIRE>(dir, g.shape, g.opt, a, grid, b->stream);
+            if (!r && b->close && gi == last_y) {
+                r = launch_close(b->d_insts, (int)b->members.size(), b->stream);
+            }
             if (timing) {
                 cudaEventRecord(e1, b->stream);
                 timing->push_back({gi, e0, e1});
@@ -654,7 +704,7 @@ int enqueue_tick(cfd_batch* b, std::vector<Timed>* timing) {
     return CFD_OK;
 }
 
-size_t member_bytes(const cfd_config& c, size_t* plane_out, int* pitch_out) {
+size_t member_bytes(const cfd_config& c, size_t* plane_out, int* pitch_out, int* slots_out) {
     int nv = cfd_nvar(c.model);
     int pitch = (c.nx + 31) / 32 * 32;
     size_t plane = (size_t)pitch * c.ny;
@@ -662,11 +712,12 @@ size_t member_bytes(const cfd_config& c, size_t* plane_out, int* pitch_out) {
     for (int s = 0; s < kNumShapesX; ++s) ty = std::max(ty, tiles_for(c.nx, c.ny, DIR_X, kShapesX[s]));
     for (int s = 0; s < kNumShapesY; ++s) ty = std::max(ty, tiles_for(c.nx, c.ny, DIR_Y, kShapesY[s]));
     ty = std::max(ty, tiles_for(c.nx, c.ny, DIR_Y, Shape{kMarchMinRows, 32}));  // shortest strips
-    int npart = std::max(ty, kInitBlocks);
+    const int slots = std::max(ty, kInitBlocks);
     size_t bytes = 4 * sizeof(float) * nv * plane  // value/compensation x 2 buffers
-                   + 256 + sizeof(DevState) + 4 * sizeof(double) * npart + 4096;
+                   + 256 + sizeof(DevState) + 4 * sizeof(double) * slots + 4096;
     if (plane_out) *plane_out = plane;
     if (pitch_out) *pitch_out = pitch;
+    if (slots_out) *slots_out = slots;
     return bytes;
 }
 
@@ -736,7 +787,7 @@ int cfd_batch_destroy(cfd_batch* b) {
 
 int cfd_batch_member_bytes(const cfd_config* cfg, size_t* bytes) {
     if (!cfg || !bytes) return cfd_fail(CFD_ERR_INVALID, "null argument");
-    *bytes = member_bytes(*cfg, nullptr, nullptr);
+    *bytes = member_bytes(*cfg, nullptr, nullptr, nullptr);
     return CFD_OK;
 }
 
@@ -768,7 +819,8 @@ static int add_member(cfd_batch* b, const cfd_config* cfg, const double* host_ic
     if (max_steps <= 0) max_steps = 0x7fffffff;
     size_t plane;
     int pitch;
-    size_t bytes = member_bytes(c, &plane, &pitch);
+    int nslots;
+    size_t bytes = member_bytes(c, &plane, &pitch, &nslots);
     if (b->used + bytes > b->budget)
         return cfd_fail(CFD_ERR_BUDGET, "instance needs %zu bytes, %zu of %zu in use", bytes,
                         b->used, b->budget);
@@ -793,9 +845,8 @@ static int add_member(cfd_batch* b, const cfd_config* cfg, const double* host_ic
             I.q2[k][w] = nv == 6 ? reinterpret_cast<float2*>(take(sizeof(float2) * plane)) : nullptr;
         }
     I.st = reinterpret_cast<DevState*>(take(sizeof(DevState)));
-    int npart = (int)((bytes - 4 * sizeof(float) * nv * plane - 256 - sizeof(DevState) - 4096) /
-                      (4 * sizeof(double)));
-    I.partials = reinterpret_cast<double*>(take(4 * sizeof(double) * npart));
+    m.nslots = nslots;
+    I.partials = reinterpret_cast<double*>(take(4 * sizeof(double) * nslots));
     I.plane = (long long)plane;
     I.pitch = pitch;
     I.nx = c.nx;

@@ -586,7 +586,7 @@ __device__ __forceinline__ void stage_read(const char* stg, int s, double* U) {
 // row k - 2 (its low-face flux applied); the raw state of row k - 1 is read
 // again from its staging slot (Euler) or carried (Allaire).
 template <int MODEL, int OPT>
-__device__ __forceinline__ void march64_strip(const MixedArgs& A, const TileGeom& g) {
+__device__ __forceinline__ void march64_strip(const MixedArgs& A, const TileGeom& g, int part) {
     using MT = ModelTraits<MODEL>;
     constexpr int NV = MT::NV;
     const int lane = threadIdx.x & 31;
@@ -600,8 +600,8 @@ __device__ __forceinline__ void march64_strip(const MixedArgs& A, const TileGeom
     const int col = g.b_org + lane;
     const bool live = col < nx;
     const int c = min(col, nx - 1);
-    const int r0 = g.a_org + 2;
-    const int r1 = min(r0 + A.rows, ny);
+    const int r0 = min(g.a_org + 2 + part * mixed::part_rows(A), ny);
+    const int r1 = min(min(r0 + mixed::part_rows(A), g.a_org + 2 + A.rows), ny);
     // the x sweep's output -> the current buffer
     const Planes64 pin = planes64<MODEL>(I, g.cur ^ 1), pout = planes64<MODEL>(I, g.cur);
     const long long pitch = I.pitch;
@@ -652,7 +652,7 @@ __device__ __forceinline__ void march64_strip(const MixedArgs& A, const TileGeom
     // Euler: unrolled by two, so that the two-row window changes roles
     // instead of being copied (y sweep 2 % faster; no change for Allaire)
 #pragma unroll(MODEL == MODEL_EULER ? 2 : 1)
-    for (int k = r0 - 2; k <= r1 + 1; ++k) {
+    for (int k = r0 < r1 ? r0 - 2 : r1 + 2; k <= r1 + 1; ++k) {
         double h[NV];
         bool neg;
         src_row(k, neg);
@@ -762,39 +762,19 @@ __device__ __forceinline__ void march64_strip(const MixedArgs& A, const TileGeom
         okp = okn;
     }
 
-    // this strip's wave speeds and masses into its slot, then the ticket
-    for (int o = 16; o > 0; o >>= 1) {
-        rmu = dmax(rmu, __shfl_down_sync(0xffffffffu, rmu, o));
-        rmv = dmax(rmv, __shfl_down_sync(0xffffffffu, rmv, o));
-        rm1 += __shfl_down_sync(0xffffffffu, rm1, o);
-        rm2 += __shfl_down_sync(0xffffffffu, rm2, o);
-    }
-    unsigned ticket = 0;
-    if (lane == 0) {
-        double* p = I.partials + 4 * g.ltile;
-        p[0] = rmu;
-        p[1] = rmv;
-        p[2] = rm1;
-        p[3] = rm2;
-        __threadfence();
-        ticket = atomicAdd(&st->ticket, 1u);
-    }
-    ticket = __shfl_sync(0xffffffffu, ticket, 0);
-    if (ticket + 1u == (unsigned)I.tiles_y) {
-        __threadfence();
-        mixed::march_finish(st, I.partials, I.tiles_y, dt);
-    }
+    mixed::march_reduce(I, g.ltile * A.split + part, rmu, rmv, rm1, rm2);
 }
 
 // Euler bounded to 128 registers for 4 CTAs per SM: its y sweep measured
 // faster than at the 3 CTAs of its unbounded register count; Allaire runs 2.
 template <int MODEL, int OPT>
 __global__ void __launch_bounds__(128, MODEL == MODEL_EULER ? 4 : 2) fast_march_kernel(MixedArgs A) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // close_steps may be scheduled
     const int gw = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int nw = gridDim.x * (blockDim.x >> 5);
-    for (int tile = gw; tile < A.ntiles; tile += nw) {
-        const TileGeom g = mixed::tile_geom<DIR_Y, mixed::kMarchMaxRows, 32>(A, tile);
-        if (!g.skip) march64_strip<MODEL, OPT>(A, g);
+    for (int w = gw; w < A.ntiles * A.split; w += nw) {
+        const TileGeom g = mixed::tile_geom<DIR_Y, mixed::kMarchMaxRows, 32>(A, w / A.split);
+        if (!g.skip) march64_strip<MODEL, OPT>(A, g, w % A.split);
     }
 }
 
@@ -820,7 +800,7 @@ __host__ __device__ constexpr int segment64_smem_bytes() {
 }
 
 template <int MODEL, int OPT>
-__device__ __forceinline__ void segment64_tile(const MixedArgs& A, const TileGeom& g) {
+__device__ __forceinline__ void segment64_tile(const MixedArgs& A, const TileGeom& g, int row_begin, int row_end) {
     using MT = ModelTraits<MODEL>;
     constexpr int NV = MT::NV;
     const int lane = threadIdx.x & 31;
@@ -848,18 +828,18 @@ __device__ __forceinline__ void segment64_tile(const MixedArgs& A, const TileGeo
     }
     src = min(max(src, 0), nx - 1);
     const bool writer = lane >= 2 && lane < 2 + mixed::kSegCells && ga < nx;
-    const int row_end = min(g.b_org + A.rows, ny);
+    row_end = min(row_end, ny);
 
     // rows staged kAhead ahead, the slot refilled at row r the one read at row r - 1
     extern __shared__ __align__(16) char seg64_stage[];
     char* stg = seg64_stage + (threadIdx.x >> 5) * (kSegSlots * stage_units<MODEL>() * 32 * 16) + 16 * lane;
 #pragma unroll
     for (int j = 0; j < kAhead; ++j) {
-        if (g.b_org + j < row_end) stage_issue<MODEL>(stg, j, pin, (g.b_org + j) * pitch + src);
+        if (row_begin + j < row_end) stage_issue<MODEL>(stg, j, pin, (row_begin + j) * pitch + src);
         mixed::cp_async_commit();
     }
     int slot = 0;
-    for (int row = g.b_org; row < row_end; ++row) {
+    for (int row = row_begin; row < row_end; ++row) {
         double h[NV];
         cp_async_wait<kAhead - 1>();  // row `row` has arrived
         stage_read<MODEL>(stg, slot, h);
@@ -935,9 +915,11 @@ template <int MODEL, int OPT>
 __global__ void __launch_bounds__(128, MODEL == MODEL_EULER ? 5 : 4) fast_segment_x_kernel(MixedArgs A) {
     const int gw = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int nw = gridDim.x * (blockDim.x >> 5);
-    for (int tile = gw; tile < A.ntiles; tile += nw) {
-        const TileGeom g = mixed::tile_geom<DIR_X, mixed::kSegCells, mixed::kSegRows>(A, tile);
-        if (!g.skip) segment64_tile<MODEL, OPT>(A, g);
+    for (int w = gw; w < A.ntiles * A.split; w += nw) {
+        const TileGeom g = mixed::tile_geom<DIR_X, mixed::kSegCells, mixed::kSegRows>(A, w / A.split);
+        if (g.skip) continue;
+        const int n = mixed::part_rows(A), r = g.b_org + (w % A.split) * n;  // this warp's rows
+        segment64_tile<MODEL, OPT>(A, g, r, min(r + n, g.b_org + A.rows));
     }
 }
 

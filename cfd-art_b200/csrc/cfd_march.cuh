@@ -23,10 +23,11 @@
 // every one.  A launch all of whose members have one such set of options runs
 // its instantiation, any other the general one.
 //
-// Reduction: each strip reduces its lanes' wave speeds and masses into its
-// own slot of the instance's partials; the strip that completes the
-// instance's ticket count combines the slots in slot order (reproducible
-// sums) and picks the instance's dt.
+// Reduction: march_reduce, close_steps.
+//
+// Where a launch's tiles leave most warps idle (small grids, where the time of
+// a sweep is that of one warp walking one tile), each tile is divided among
+// several warps: A.split.
 //
 // Warp segments (the x sweep, further down): the lanes hold 32 consecutive
 // cells of a row and exchange neighbour values by shuffles.
@@ -58,40 +59,112 @@ __device__ __forceinline__ void march_rotate_in(float* h, float* l, bool neg) {
     l[MT::IT] = -tl;
 }
 
-// Last-strip finish of the wave-speed reduction, by one warp: slots in slot
-// order per lane, then a fixed shuffle tree (reproducible sums).
-__device__ __forceinline__ void march_finish(DevState* st, const double* partials, int nslots,
-                                             double dt_used) {
-    const int lane = threadIdx.x & 31;
-    double mu = 0.0, mv = 0.0, m1 = 0.0, m2 = 0.0;
-    for (int b = lane; b < nslots; b += 32) {
-        mu = smax(mu, __ldcg(partials + 4 * b + 0));
-        mv = smax(mv, __ldcg(partials + 4 * b + 1));
-        m1 += __ldcg(partials + 4 * b + 2);
-        m2 += __ldcg(partials + 4 * b + 3);
-    }
+// The warp's four sums of a slot's lanes (speeds by maximum), fixed shuffle
+// tree: reproducible sums, in lane 0.
+__device__ __forceinline__ void warp_sums(double& mu, double& mv, double& m1, double& m2) {
     for (int o = 16; o > 0; o >>= 1) {
         mu = smax(mu, __shfl_down_sync(0xffffffffu, mu, o));
         mv = smax(mv, __shfl_down_sync(0xffffffffu, mv, o));
         m1 += __shfl_down_sync(0xffffffffu, m1, o);
         m2 += __shfl_down_sync(0xffffffffu, m2, o);
     }
-    if (lane == 0) {
-        DevState s = *st;
-        s.t = s.t + dt_used;
-        s.n = s.n + 1;
-        if (fabs(s.t - s.T) < 1e-12) s.t = s.T;
-        s.maxu = mu;
-        s.maxv = mv;
-        s.mass1 = m1 * s.dx * s.dy;
-        s.mass2 = m2 * s.dx * s.dy;
-        s.dt = choose_dt(s, mu, mv);
-        s.done = !(s.t < s.T);
-        s.ticket = 0;
-        *st = s;
-        __threadfence();
-    }
 }
+__device__ __forceinline__ void put_slot(double* p, double mu, double mv, double m1, double m2) {
+    reinterpret_cast<double2*>(p)[0] = make_double2(mu, mv);
+    reinterpret_cast<double2*>(p)[1] = make_double2(m1, m2);
+}
+__device__ __forceinline__ void add_slot(const double* p, double& mu, double& mv, double& m1, double& m2) {
+    const double2 a = __ldcg(reinterpret_cast<const double2*>(p));
+    const double2 b = __ldcg(reinterpret_cast<const double2*>(p) + 1);
+    mu = smax(mu, a.x);
+    mv = smax(mv, a.y);
+    m1 += b.x;
+    m2 += b.y;
+}
+
+// Closes a member's step with the reduced wave speeds and masses of its new
+// state: time, step count, dt of the next step.
+__device__ __forceinline__ void close_step(DevState* st, double mu, double mv, double m1, double m2) {
+    DevState s = *st;
+    s.t = s.t + s.dt;
+    s.n = s.n + 1;
+    if (fabs(s.t - s.T) < 1e-12) s.t = s.T;
+    s.maxu = mu;
+    s.maxv = mv;
+    s.mass1 = m1 * s.dx * s.dy;
+    s.mass2 = m2 * s.dx * s.dy;
+    s.dt = choose_dt(s, mu, mv);
+    s.done = !(s.t < s.T);
+    s.ticket = 0;
+    *st = s;
+    __threadfence();
+}
+
+// A part's wave speeds and masses (per lane) into its slot, by its warp.  The
+// warp that completes the member's slots combines them in slot order
+// (reproducible sums) and closes the step; a member of many slots is closed by
+// close_steps instead, launched behind the y sweeps: the fence and the ticket
+// of every part and one warp's walk over the slots took 10.5 us of the 63 us
+// sweep of a 2048^2 Euler member (2,368 slots); sweep and close together take
+// 57.6.  At 256^2 (1,024 slots) a step takes 14.1 us with the close and 16.2
+// with the ticket; up to kTicketSlots, one per lane, the ticket is as fast
+// (64^2: 10.3 and 10.4).  Batches of many uneven members that fit one round of
+// the resident warps hide the ticket (24 members 69.9 us, 71.3 with the close),
+// those of several rounds do not (100 members 363, 336).
+__device__ __forceinline__ void march_reduce(const Inst& I, int slot, double mu, double mv, double m1,
+                                             double m2) {
+    const int lane = threadIdx.x & 31;
+    DevState* st = I.st;
+    warp_sums(mu, mv, m1, m2);
+    if (lane == 0) put_slot(I.partials + 4 * slot, mu, mv, m1, m2);
+    if (I.closed) return;
+    unsigned t = 0;
+    if (lane == 0) {
+        __threadfence();
+        t = atomicAdd(&st->ticket, 1u);
+    }
+    if (__shfl_sync(0xffffffffu, t, 0) + 1u != (unsigned)I.slots) return;
+    __threadfence();
+    mu = mv = m1 = m2 = 0.0;
+    if (lane < I.slots) add_slot(I.partials + 4 * lane, mu, mv, m1, m2);
+    warp_sums(mu, mv, m1, m2);
+    if (lane == 0) close_step(st, mu, mv, m1, m2);
+}
+
+// Closes the steps of the members marked so, a CTA each, from the slots their
+// y sweep has filled; members that sweep skipped are skipped.
+constexpr int kCloseThreads = 256;
+constexpr int kTicketSlots = 32;  // most slots of a member closed by its last warp, one per lane
+__global__ void __launch_bounds__(kCloseThreads) close_steps(const Inst* insts) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // the last y sweep's completion
+    const Inst& I = insts[blockIdx.x];
+    DevState* st = I.st;
+    if (!I.closed || !I.active || st->done || st->n >= I.max_steps) return;
+    double mu = 0.0, mv = 0.0, m1 = 0.0, m2 = 0.0;
+    const int n = I.slots;
+    const double* p = I.partials;
+#pragma unroll 4
+    for (int b = threadIdx.x; b < n; b += kCloseThreads) add_slot(p + 4 * b, mu, mv, m1, m2);
+    warp_sums(mu, mv, m1, m2);
+    __shared__ __align__(16) double red[4 * (kCloseThreads / 32)];
+    if ((threadIdx.x & 31) == 0) put_slot(red + 4 * (threadIdx.x >> 5), mu, mv, m1, m2);
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    for (int w = 1; w < kCloseThreads / 32; ++w) {
+        const double* q = red + 4 * w;
+        mu = smax(mu, q[0]);
+        mv = smax(mv, q[1]);
+        m1 += q[2];
+        m2 += q[3];
+    }
+    close_step(st, mu, mv, m1, m2);
+}
+
+// Parts of a tile: `rows` rows divided into A.split, a warp each.  Undivided,
+// a 64^2 grid is 18 tiles of 12 rows in x and 8 strips of 16 (20 with the halo)
+// in y, one warp walking each: 17.4 us a step of Euler, 10.2 divided; 256^2
+// 19.9 -> 14.0 us (fast FP64 25.9 -> 16.9).
+__device__ __forceinline__ int part_rows(const MixedArgs& A) { return (A.rows + A.split - 1) / A.split; }
 
 // Rows staged through shared memory with cp.async (no registers held by the
 // loads in flight): a ring of kMSlots slots per lane holding at least rows
@@ -150,10 +223,10 @@ __host__ __device__ constexpr int sweep_options(int flags) {
     return flags & MF_GODUNOV ? flags & MF_OPTIONS & ~3 : flags & MF_OPTIONS;
 }
 
-// One strip: rows [r0, r1) of the columns [b_org, b_org + 32) of instance
-// g.inst.
+// One part of a strip: rows [r0, r1) of the columns [b_org, b_org + 32) of
+// instance g.inst (none where the strip is shorter than its parts).
 template <int MODEL, int OPT>
-__device__ __forceinline__ void march_strip(const MixedArgs& A, const TileGeom& g) {
+__device__ __forceinline__ void march_strip(const MixedArgs& A, const TileGeom& g, int part) {
     using MT = ModelTraits<MODEL>;
     constexpr int NV = MT::NV;
     const int lane = threadIdx.x & 31;
@@ -169,8 +242,8 @@ __device__ __forceinline__ void march_strip(const MixedArgs& A, const TileGeom& 
     const int col = g.b_org + lane;
     const bool live = col < nx;
     const int c = min(col, nx - 1);
-    const int r0 = g.a_org + 2;
-    const int r1 = min(r0 + A.rows, ny);
+    const int r0 = min(g.a_org + 2 + part * part_rows(A), ny);
+    const int r1 = min(min(r0 + part_rows(A), g.a_org + 2 + A.rows), ny);
     // the y sweep reads the x sweep's output.  Euler holds the planes in
     // registers (2 % faster); Allaire, at its 128-register limit, spilled that
     // way and measured 3 % slower, so it reads them from the member descriptor
@@ -349,7 +422,7 @@ __device__ __forceinline__ void march_strip(const MixedArgs& A, const TileGeom& 
             zs_low = MODEL == MODEL_ALLAIRE ? Fh[NV + 1] : 0.f;
         }
     };
-    int k = r0 - 2;
+    int k = r0 < r1 ? r0 - 2 : r1 + 2;
     while (k <= r1 + 1) {
         row_step(k, Bool<false>{});
         ++k;
@@ -362,29 +435,7 @@ __device__ __forceinline__ void march_strip(const MixedArgs& A, const TileGeom& 
             for (; k + kMAhead < r1; ++k) row_step(k, Bool<true>{});
     }
 
-    // this strip's wave speeds and masses into its slot, then the ticket
-    double mu = (double)rmu, mv = (double)rmv;
-    for (int o = 16; o > 0; o >>= 1) {
-        mu = smax(mu, __shfl_down_sync(0xffffffffu, mu, o));
-        mv = smax(mv, __shfl_down_sync(0xffffffffu, mv, o));
-        rm1 += __shfl_down_sync(0xffffffffu, rm1, o);
-        rm2 += __shfl_down_sync(0xffffffffu, rm2, o);
-    }
-    unsigned ticket = 0;
-    if (lane == 0) {
-        double* p = I.partials + 4 * g.ltile;
-        p[0] = mu;
-        p[1] = mv;
-        p[2] = rm1;
-        p[3] = rm2;
-        __threadfence();
-        ticket = atomicAdd(&st->ticket, 1u);
-    }
-    ticket = __shfl_sync(0xffffffffu, ticket, 0);
-    if (ticket + 1u == (unsigned)I.tiles_y) {
-        __threadfence();
-        march_finish(st, I.partials, I.tiles_y, dt);
-    }
+    march_reduce(I, g.ltile * A.split + part, (double)rmu, (double)rmv, rm1, rm2);
 }
 
 // Persistent sweep: warp w of the W warps of the grid walks the strips w,
@@ -393,11 +444,12 @@ __device__ __forceinline__ void march_strip(const MixedArgs& A, const TileGeom& 
 // some of them.
 template <int MODEL, int OPT>
 __global__ void __launch_bounds__(128, 4) mixed_march_kernel(MixedArgs A) {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");  // close_steps may be scheduled
     const int gw = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int nw = gridDim.x * (blockDim.x >> 5);
-    for (int tile = gw; tile < A.ntiles; tile += nw) {
-        const TileGeom g = tile_geom<DIR_Y, kMarchMaxRows, 32>(A, tile);
-        if (!g.skip) march_strip<MODEL, OPT>(A, g);
+    for (int w = gw; w < A.ntiles * A.split; w += nw) {
+        const TileGeom g = tile_geom<DIR_Y, kMarchMaxRows, 32>(A, w / A.split);
+        if (!g.skip) march_strip<MODEL, OPT>(A, g, w % A.split);
     }
 }
 
@@ -434,7 +486,7 @@ __device__ __forceinline__ void shfl_down_n(const float* x, float* y) {
 }
 
 template <int MODEL, int OPT>
-__device__ __forceinline__ void segment_tile(const MixedArgs& A, const TileGeom& g) {
+__device__ __forceinline__ void segment_tile(const MixedArgs& A, const TileGeom& g, int row_begin, int row_end) {
     using MT = ModelTraits<MODEL>;
     constexpr int NV = MT::NV;
     const int lane = threadIdx.x & 31;
@@ -464,23 +516,23 @@ __device__ __forceinline__ void segment_tile(const MixedArgs& A, const TileGeom&
     }
     src = min(max(src, 0), nx - 1);
     const bool writer = lane >= 2 && lane < 2 + kSegCells && ga < nx;
-    const int row_end = min(g.b_org + A.rows, ny);
+    row_end = min(row_end, ny);
 
     extern __shared__ __align__(16) char seg_stage[];
     constexpr int MU = march_units<MODEL>();
     constexpr int SB = MU * 32 * 16;
     static_assert((kSSlots & (kSSlots - 1)) == 0, "a power of two");
     char* stg = seg_stage + (threadIdx.x >> 5) * (kSSlots * SB) + 16 * lane;
-    unsigned off_in = (unsigned)g.b_org * pitch + src;           // the next row to load
-    unsigned off_out = (unsigned)g.b_org * pitch + (unsigned)ga;  // this row's cell
+    unsigned off_in = (unsigned)row_begin * pitch + src;           // the next row to load
+    unsigned off_out = (unsigned)row_begin * pitch + (unsigned)ga;  // this row's cell
 #pragma unroll
     for (int j = 0; j < kMAhead; ++j) {
-        if (g.b_org + j < row_end) mstage_issue<MODEL>(stg + j * SB, qin, off_in);
+        if (row_begin + j < row_end) mstage_issue<MODEL>(stg + j * SB, qin, off_in);
         off_in += pitch;
         cp_async_commit();
     }
     int at = 0;
-    for (int row = g.b_org; row < row_end; ++row, off_in += pitch, off_out += pitch, ++at) {
+    for (int row = row_begin; row < row_end; ++row, off_in += pitch, off_out += pitch, ++at) {
         float h[NV], l[NV];
         asm volatile("cp.async.wait_group %0;\n" ::"n"(kMAhead - 1) : "memory");
         mstage_read<MODEL>(stg + (unsigned)(at & (kSSlots - 1)) * SB, h, l);
@@ -588,9 +640,11 @@ __global__ void __launch_bounds__(128, MODEL == MODEL_EULER ? 8 : 5)
     mixed_segment_x_kernel(MixedArgs A) {
     const int gw = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const int nw = gridDim.x * (blockDim.x >> 5);
-    for (int tile = gw; tile < A.ntiles; tile += nw) {
-        const TileGeom g = tile_geom<DIR_X, kSegCells, kSegRows>(A, tile);
-        if (!g.skip) segment_tile<MODEL, OPT>(A, g);
+    for (int w = gw; w < A.ntiles * A.split; w += nw) {
+        const TileGeom g = tile_geom<DIR_X, kSegCells, kSegRows>(A, w / A.split);
+        if (g.skip) continue;
+        const int n = part_rows(A), r = g.b_org + (w % A.split) * n;  // this warp's rows
+        segment_tile<MODEL, OPT>(A, g, r, min(r + n, g.b_org + A.rows));
     }
 }
 

@@ -55,10 +55,11 @@ struct Inst {
     // 1/(g1 - 1), 1/(g2 - 1), g1 p1/(g1 - 1), g2 p2/(g2 - 1)
     double pd[4];
     DevState* st;
-    double* partials;   // 4 per y tile
+    double* partials;   // 4 per y tile (marching: per strip part)
     int tiles_x, tiles_y;   // tiles of each sweep
     int max_steps;          // stop after this many steps (and at t >= T)
     int active;             // 0: skip
+    int slots, closed;      // marching y sweep: reduction slots in use; 1: closed by close_steps
     int fp64;               // 1: the planes hold FP64 values (fast FP64 form, cfd_fast64.cuh)
 };
 
@@ -77,8 +78,10 @@ struct MixedArgs {
     const TileEnt* tiles;   // tiles of this launch
     int ntiles;             // tiles of this launch
     int chunk;              // CTA c walks tiles [c * chunk, (c + 1) * chunk) (persistent)
-    int rows;               // marching strips: cells along the sweep per strip
+    int rows;               // warp sweeps: rows of a tile
+    int split;              // warp sweeps: parts a tile is divided into, a warp each (2^n)
 };
+
 
 // Per-tile constants held in registers (one vector load per tile instead of
 // a global load at every use).
