@@ -33,3 +33,20 @@ def test_divided_small_grid_equals_undivided(prec, recipe, nx, ny):
     assert np.array_equal(alone, mixed)
     # the mass sums are grouped by strip: equal to the rounding of their sums
     assert abs(st.mass1 - st2.mass1) <= 1e-12 * abs(st.mass1)
+
+
+@pytest.mark.parametrize("prec", [G.MIXED, G.FP64_FAST], ids=["mixed", "fast"])
+def test_replayed_ticks_equal_ticks_launched_one_by_one(prec):
+    """31 ticks are launched one by one, 32 and more in one call replay a
+    graph, and so do later calls of 8; the states are the same."""
+    cfg = G.recipe_config("shock_bubbles", 40, 33)
+    cfg.precision = prec
+    states = []
+    for calls in [(31, 33), (1,) * 64, (64,), (7,) * 8 + (8,), (40, 8, 8, 8)]:
+        with G.Batch() as b:
+            m = b.add_recipe(cfg, "shock_bubbles", max_steps=64)
+            for ticks in calls:
+                b.step(ticks)
+            st = b.status(m)
+            states.append((st.n, st.t, st.mass1, b.download(m).tobytes()))
+    assert states[0][0] == 64 and all(s == states[0] for s in states)
