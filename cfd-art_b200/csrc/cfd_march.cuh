@@ -135,11 +135,11 @@ __device__ __forceinline__ void march_reduce(const Inst& I, int slot, double mu,
 // y sweep has filled; members that sweep skipped are skipped.
 constexpr int kCloseThreads = 256;
 constexpr int kTicketSlots = 32;  // most slots of a member closed by its last warp, one per lane
-__global__ void __launch_bounds__(kCloseThreads) close_steps(const Inst* insts) {
+__global__ void __launch_bounds__(kCloseThreads) close_steps(const Inst* insts, int which) {
     asm volatile("griddepcontrol.wait;" ::: "memory");  // the last y sweep's completion
     const Inst& I = insts[blockIdx.x];
     DevState* st = I.st;
-    if (!I.closed || !I.active || st->done || st->n >= I.max_steps) return;
+    if (I.closed != which || !I.active || st->done || st->n >= I.max_steps) return;
     double mu = 0.0, mv = 0.0, m1 = 0.0, m2 = 0.0;
     const int n = I.slots;
     const double* p = I.partials;

@@ -59,7 +59,7 @@ struct Inst {
     int tiles_x, tiles_y;   // tiles of each sweep
     int max_steps;          // stop after this many steps (and at t >= T)
     int active;             // 0: skip
-    int slots, closed;      // marching y sweep: reduction slots in use; 1: closed by close_steps
+    int slots, closed;      // marching y sweep: reduction slots in use; the close_steps launch that closes it (0: its last warp)
     int fp64;               // 1: the planes hold FP64 values (fast FP64 form, cfd_fast64.cuh)
 };
 

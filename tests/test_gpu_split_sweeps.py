@@ -50,3 +50,36 @@ def test_replayed_ticks_equal_ticks_launched_one_by_one(prec):
             st = b.status(m)
             states.append((st.n, st.t, st.mass1, b.download(m).tobytes()))
     assert states[0][0] == 64 and all(s == states[0] for s in states)
+
+
+@pytest.mark.parametrize("ticks", [(1, 2, 17), (70,)], ids=["launched", "replayed"])
+@pytest.mark.parametrize("sizes", [[(40, 33)] * 4, [(300, 200), (5, 3), (1024, 700), (64, 64)]],
+                         ids=["small", "uneven"])
+def test_models_and_forms_side_by_side_equal_each_alone(sizes, ticks):
+    """Chains of launches of different models and forms run at the same time."""
+    members = []
+    for (nx, ny), (recipe, prec) in zip(sizes, [("shock_bubbles", G.MIXED),
+                                                ("water_shock_air_bubble", G.FP64_FAST),
+                                                ("water_shock_air_bubble", G.MIXED),
+                                                ("shock_bubbles", G.FP64_FAST)]):
+        cfg = G.recipe_config(recipe, nx, ny)
+        cfg.precision = prec
+        members.append((cfg, recipe))
+
+    def solve(some):
+        with G.Batch() as b:
+            ids = [b.add_recipe(c, r, max_steps=sum(ticks) - 3 * k)
+                   for k, (c, r) in some]
+            for n in ticks:
+                b.step(n)
+            out = []
+            for i in ids:
+                st = b.status(i)
+                out.append((st.n, st.t, st.mass1, st.maxu, st.maxv, b.download(i).tobytes()))
+            return out
+
+    numbered = list(enumerate(members))
+    together = solve(numbered)
+    for k, m in numbered:
+        assert together[k][0] == sum(ticks) - 3 * k
+        assert together[k] == solve([(k, m[:2])])[0]
