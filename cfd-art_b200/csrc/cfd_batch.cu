@@ -440,7 +440,22 @@ struct Member {
 // kMinPartRows rows beside its 4 halo rows.
 constexpr int kSplitWarps = 16, kMinPartRows = 2;
 
-constexpr int kSides = 3;  // of the four (model, form) chains, those beside the first
+// The unfinished members of a (model, form) step in up to kStrands strands, the
+// chains of launches of a tick (enqueue_ticks), from strand_cells cells on.
+// Beside one another the sweeps of one strand fill the start and the end of
+// another's: a tick of 24 uneven mixed Euler members (1.7e6 cells) takes 53.8 us
+// in one strand, 51.0 in two, 49.4 in three and 49.9 in four; 8 of 1024^2
+// 211 -> 172, 100 small ones 141 -> 118; fast FP64 82 -> 76, 298 -> 261 and
+// 210 -> 178.  Smaller sums lose to the launches (6 members of 1.3e5 cells
+// 15.8 -> 16.4 us).  The mixed two-material sweeps are both bound by
+// instruction issue: 24 members 96 -> 103 us, 8 of 512^2 the same, gains only
+// where a sweep has several rounds of warps (8 of 1024^2 352 -> 325).
+constexpr int kStrands = 3;
+long long strand_cells(int model, int fp64) {
+    return model == CFD_MODEL_ALLAIRE && !fp64 ? 3000000 : 700000;
+}
+
+constexpr int kSides = 4 * kStrands - 1;  // strands beside the first
 
 }  // namespace
 
@@ -462,10 +477,10 @@ struct cfd_batch {
         int split; // warp sweeps: parts (warps) per tile
         int close; // y: Inst::closed of the members whose steps close_steps closes; 0: none
     };
-    // the x and the y launch of each (model, form) with unfinished members, in
-    // pairs: the chains of launches of a tick, which share no member
+    // the x and the y launch of each strand of unfinished members of one model
+    // and form, in pairs
     std::vector<Group> groups;
-    cudaStream_t side[kSides] = {};  // the chains beside the first (created when first used)
+    cudaStream_t side[kSides] = {};  // the strands beside the first (created when first used)
     cudaEvent_t fork = nullptr, join[kSides] = {};
     bool dirty = true;
     // [model][dir]; y sweeps march by default (measured fastest on B200 for
@@ -565,10 +580,33 @@ int build_tables(cfd_batch* b) {
         return (long long)b->members[x].cfg.nx * b->members[x].cfg.ny >
                (long long)b->members[y].cfg.nx * b->members[y].cfg.ny;
     });
+    // each member's strand: the one with the fewest cells so far
+    std::vector<int> strand_of(b->members.size(), 0);
+    int strands[2][2];
+    for (int model = 0; model < 2; ++model)
+        for (int f64 = 0; f64 < 2; ++f64) {
+            long long cells = 0, in_strand[kStrands] = {};
+            std::vector<int> mine;
+            for (int i : order) {
+                const Member& m = b->members[i];
+                if (m.cfg.model != model || m.inst.fp64 != f64 || m.final) continue;
+                mine.push_back(i);
+                cells += (long long)m.cfg.nx * m.cfg.ny;
+            }
+            int& n = strands[model][f64];
+            n = cells < strand_cells(model, f64) ? 1 : kStrands;
+            n = std::max(1, std::min(n, (int)mine.size()));
+            for (int i : mine) {
+                const int k = (int)(std::min_element(in_strand, in_strand + n) - in_strand);
+                strand_of[i] = k;
+                in_strand[k] += (long long)b->members[i].cfg.nx * b->members[i].cfg.ny;
+            }
+        }
     std::vector<TileEnt> all;
     for (int model = 0; model < 2; ++model)
         for (int f64 = 0; f64 < 2; ++f64)
-            for (int dir = 0; dir < 2; ++dir) {
+            for (int sd = 0; sd < 2 * strands[model][f64]; ++sd) {
+                const int strand = sd / 2, dir = sd % 2;
                 cfd_batch::Group g;
                 g.model = model;
                 g.fp64 = f64;
@@ -583,6 +621,7 @@ int build_tables(cfd_batch* b) {
                     const Member& m = b->members[idx];
                     // finished members have no tiles
                     if (m.cfg.model != model || m.inst.fp64 != f64 || m.final) continue;
+                    if (strand_of[idx] != strand) continue;
                     const int len = dir == DIR_X ? m.cfg.nx : m.cfg.ny;
                     const int wid = dir == DIR_X ? m.cfg.ny : m.cfg.nx;
                     const int along = (len + sh.ts - 1) / sh.ts;
@@ -605,7 +644,7 @@ int build_tables(cfd_batch* b) {
                 g.split = 1;
                 g.close = 0;
                 if (dir == DIR_X || g.shape == kMarchShape)
-                    while (g.ntiles * g.split * 2 <= kSplitWarps * b->sms &&
+                    while (g.ntiles * strands[model][f64] * g.split * 2 <= kSplitWarps * b->sms &&
                            g.rows >= g.split * 2 * (dir == DIR_X ? 1 : kMinPartRows) &&
                            (dir == DIR_X || slots * g.split * 2 <= 1.0))
                         g.split *= 2;
@@ -613,9 +652,10 @@ int build_tables(cfd_batch* b) {
                     for (int idx : order) {
                         const Member& m = b->members[idx];
                         if (m.cfg.model != model || m.inst.fp64 != f64 || m.final) continue;
+                        if (strand_of[idx] != strand) continue;
                         insts[idx].slots = insts[idx].tiles_y * g.split;
                         const bool closed = insts[idx].slots > kTicketSlots;
-                        insts[idx].closed = closed ? 1 + 2 * model + f64 : 0;
+                        insts[idx].closed = closed ? 1 + (2 * model + f64) * kStrands + strand : 0;
                         if (closed) g.close = insts[idx].closed;
                     }
                 if (g.ntiles) b->groups.push_back(g);
@@ -673,10 +713,10 @@ int launch_close(const Inst* insts, int members, int which, cudaStream_t st) {
     return CFD_OK;
 }
 
-// The x and y launches of a tick of chain `chain` (groups 2 chain and
-// 2 chain + 1), and the close of its members' steps.
-int enqueue_chain(cfd_batch* b, int chain, cudaStream_t st, std::vector<Timed>* timing) {
-    for (int gi = 2 * chain; gi < 2 * chain + 2; ++gi) {
+// The x and y launches of a tick of strand `k` (groups 2 k and 2 k + 1), and
+// the close of its members' steps.
+int enqueue_strand(cfd_batch* b, int k, cudaStream_t st, std::vector<Timed>* timing) {
+    for (int gi = 2 * k; gi < 2 * k + 2; ++gi) {
         const auto& g = b->groups[gi];
         MixedArgs a;
         a.insts = b->d_insts;
@@ -708,7 +748,7 @@ int enqueue_chain(cfd_batch* b, int chain, cudaStream_t st, std::vector<Timed>* 
     return CFD_OK;
 }
 
-// The side streams and events of `n` chains; false (and serial launches) if
+// The side streams and events of `n` strands; false (and serial launches) if
 // one cannot be made.
 bool have_sides(cfd_batch* b, int n) {
     auto event = [](cudaEvent_t& e) {
@@ -723,29 +763,29 @@ bool have_sides(cfd_batch* b, int n) {
     return ok;
 }
 
-// Queues `n` ticks on the batch stream (or on its capture).  Chains of
-// different (model, form) share no member, so each runs on its own stream
-// between a fork and a join per call: one chain's sweeps fill the warps that
-// another's last tiles and short launches leave idle, and an x sweep (bound by
+// Queues `n` ticks on the batch stream (or on its capture).  Strands share
+// no member, so each runs on its own stream between a fork and a join per
+// call: one strand's sweeps fill the warps that another's last tiles and
+// short launches leave idle, and an x sweep (bound by
 // memory) a y sweep's (bound by instruction issue).  A tick of Euler 2048^2
 // beside Allaire 2048x1024, mixed: 201 us one after the other, 169 beside one
 // another; Euler 2048^2 mixed and fast FP64 254 -> 214; four 512^2 members
 // of all kinds 87 -> 51; four 64^2 41.6 -> 15.6 (launched one by one 60 -> 43).
 // With `timing` the launches follow one another on the batch stream.
 int enqueue_ticks(cfd_batch* b, int n, std::vector<Timed>* timing) {
-    const int chains = (int)b->groups.size() / 2;
+    const int strands = (int)b->groups.size() / 2;
     int r = CFD_OK;
-    if (timing || chains < 2 || !have_sides(b, chains)) {
+    if (timing || strands < 2 || !have_sides(b, strands)) {
         for (int i = 0; i < n; ++i)
-            for (int c = 0; c < chains && !r; ++c) r = enqueue_chain(b, c, b->stream, timing);
+            for (int c = 0; c < strands && !r; ++c) r = enqueue_strand(b, c, b->stream, timing);
         return r;
     }
     BTRY(cudaEventRecord(b->fork, b->stream));
-    for (int c = 1; c < chains; ++c) BTRY(cudaStreamWaitEvent(b->side[c - 1], b->fork, 0));
+    for (int c = 1; c < strands; ++c) BTRY(cudaStreamWaitEvent(b->side[c - 1], b->fork, 0));
     for (int i = 0; i < n && !r; ++i)
-        for (int c = 0; c < chains && !r; ++c)
-            r = enqueue_chain(b, c, c ? b->side[c - 1] : b->stream, nullptr);
-    for (int c = 1; c < chains; ++c) {  // also after a failed launch: nothing runs on unjoined
+        for (int c = 0; c < strands && !r; ++c)
+            r = enqueue_strand(b, c, c ? b->side[c - 1] : b->stream, nullptr);
+    for (int c = 1; c < strands; ++c) {  // also after a failed launch: nothing runs on unjoined
         BTRY(cudaEventRecord(b->join[c - 1], b->side[c - 1]));
         BTRY(cudaStreamWaitEvent(b->stream, b->join[c - 1], 0));
     }

@@ -83,3 +83,29 @@ def test_models_and_forms_side_by_side_equal_each_alone(sizes, ticks):
     for k, m in numbered:
         assert together[k][0] == sum(ticks) - 3 * k
         assert together[k] == solve([(k, m[:2])])[0]
+
+
+@pytest.mark.parametrize("ticks", [(5, 12), (40,)], ids=["launched", "replayed"])
+@pytest.mark.parametrize("recipe,prec", [("shock_bubbles", G.MIXED), ("shock_bubbles", G.FP64_FAST),
+                                         ("water_shock_air_bubble", G.FP64_FAST)])
+def test_strands_of_one_form_equal_each_member_alone(recipe, prec, ticks):
+    """7.7e5 cells in all step in three strands, one member finishing early."""
+    members = []
+    for k, (nx, ny) in enumerate([(64, 64), (700, 500), (300, 411), (512, 512), (129, 257)]):
+        cfg = G.recipe_config(recipe, nx, ny)
+        cfg.precision = prec
+        members.append((cfg, sum(ticks) - 9 * (k == 2)))
+
+    def solve(some):
+        with G.Batch() as b:
+            ids = [b.add_recipe(c, recipe, max_steps=n) for c, n in some]
+            for n in ticks:
+                b.step(n)
+            return [(b.status(i), b.download(i)) for i in ids]
+
+    for (st, grid), m in zip(solve(members), members):
+        st1, alone = solve([m])[0]
+        assert st.n == st1.n == m[1]
+        assert (st.t, st.maxu, st.maxv) == (st1.t, st1.maxu, st1.maxv)
+        assert np.array_equal(grid, alone)
+        assert abs(st.mass1 - st1.mass1) <= 1e-12 * abs(st1.mass1)
