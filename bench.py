@@ -519,7 +519,7 @@ def bench_single(args, ctx, G, stream, clocks):
     else:
         mx, my, n = s.step_timed(4)
         st = s.status(mid)
-        launches = 2 * K
+        launches = n // 4 * K
         dom = 0 if mx >= my else 1
         kname = "fast_sweep" if prec == "fp64_fast" else "mixed_sweep"
         rl = roofline([f"{kname}_x", f"{kname}_y"][dom], [mx, my][dom], 4,
@@ -703,7 +703,7 @@ def bench_batch(args, ctx, G, stream, clocks):
                        "autotune_steps": sum(pre.values()), "graph": "8 ticks per CUDA graph",
                        "l2": f"state {cells * 32 / 1e6:.0f} MB > 126 MB L2, no flush",
                        "parallelism": f"replicas x{ctx.world}"},
-            "clocks": ck, "gpu_launches": 2 * K, "roofline": rl, "e2e": e2e,
+            "clocks": ck, "gpu_launches": n // 4 * K, "roofline": rl, "e2e": e2e,
             "sim": {"cell_updates_timed": upd}}
 
 
