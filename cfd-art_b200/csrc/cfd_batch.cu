@@ -1,13 +1,14 @@
 // Batched solves: many independent grids of uneven sizes advanced together.
 //
 // A batch owns device state for each member solve (instance) and advances
-// all active instances by one split step per "tick": one persistent x-sweep
-// launch and one persistent y-sweep launch per model present, over a tile
-// list that covers every active instance (x: warp segments, csrc/cfd_march.cuh;
-// y: shared-memory tiles, csrc/cfd_mixed.cuh, or marching strips).  Each instance
-// keeps its own time-loop state (n, t, dt, T, max_steps), picks its own dt
-// after each step and stops on its own.  Ticks are captured into a CUDA graph
-// that is replayed until the membership changes.  Instances are admitted
+// all active instances by one split step per "tick": an x-sweep and a y-sweep
+// launch per strand (members of one model and precision form; several strands
+// step beside one another, enqueue_ticks), over a tile list that covers the
+// strand's active instances (x: warp segments, csrc/cfd_march.cuh; y: shared-memory
+// tiles, csrc/cfd_mixed.cuh, or marching strips).  Each instance keeps its own
+// time-loop state (n, t, dt, T, max_steps), picks its own dt after each step
+// and stops on its own.  Ticks are captured into a CUDA graph, replayed until
+// the membership changes, once enough of them pay for it.  Instances are admitted
 // against a device-memory budget, so a server can keep adding work while
 // others run.
 //
@@ -139,11 +140,16 @@ int warp_per_sm(int model, int fp64, int dir, int opt) {
     return n;
 }
 
-// Persistent launch: as many warps as fit on the device (never more than
-// there are tiles), each walking every W-th tile.
+// y sweeps: a persistent launch of as many warps as fit on the device (never
+// more than there are tiles), each walking every W-th tile, since a strip pays for its
+// halo rows and its setup.  x sweeps: a warp per tile, handed out as warps
+// finish, since their rows differ in cost (fallbacks, memory): Euler 2900^2 mixed
+// 106.9 us persistent, 99.4 so; fast FP64 141.8 -> 132.4 and 2048^2 75.1 -> 73.0;
+// y launched so 109.5 -> 116.3.
 int launch_warp(int model, int fp64, int dir, int opt, const MixedArgs& a, int sms, cudaStream_t st) {
     const WarpKernel k = warp_kernel(model, fp64, dir, opt);
-    const int warps = std::max(1, std::min(a.ntiles * a.split, warp_per_sm(model, fp64, dir, opt) * sms * 4));
+    const int fit = warp_per_sm(model, fp64, dir, opt) * sms * 4;
+    const int warps = std::max(1, dir == DIR_X ? a.ntiles * a.split : std::min(a.ntiles * a.split, fit));
     k.fn<<<(warps + 3) / 4, 128, k.smem, st>>>(a);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cfd_fail(CFD_ERR_CUDA, "sweep launch: %s", cudaGetErrorString(e));
@@ -191,14 +197,24 @@ int march_rows(const std::vector<std::pair<int, int>>& grids, long long slots) {
 // other, each costing its rows plus about two rows' worth of setup (the
 // member's constants, the first row's load), so the count with the fewest
 // (rounds x (rows + 2)) is taken, the largest on ties.  A lone grid that
-// leaves resident warps idle at 32 rows gets shorter tiles.
+// leaves resident warps idle at 32 rows gets shorter tiles.  From two rounds
+// of tiles of kManyRows on rounds no longer matter (launch_warp): at 2900^2
+// the rule's 28 to 32 rows take 99.4 us (Euler mixed), 132.4 (fast) and 210.3
+// (Allaire fast, 2048^2 115.2), 20 rows 93.2, 132.6 and 212.7 (115.5), 16 rows
+// 91.9, 132.5 and 210.7 (113.3), but Allaire mixed 2048^2 83.4 against 81.3.
 int seg_rows(const std::vector<std::pair<int, int>>& grids, long long slots) {
     int best = kSegRows;
     long long best_cost = -1;
-    for (int rows = kSegRows; rows >= kSegMinRows; rows -= 2) {
+    auto tiles_of = [&](int rows) {
         long long tiles = 0;
         for (const auto& g : grids)
             tiles += (long long)((g.first + kSegCells - 1) / kSegCells) * ((g.second + rows - 1) / rows);
+        return tiles;
+    };
+    constexpr int kManyRows = 20;
+    if (tiles_of(kManyRows) >= 2 * slots) return kManyRows;
+    for (int rows = kSegRows; rows >= kSegMinRows; rows -= 2) {
+        const long long tiles = tiles_of(rows);
         if (!tiles) return kSegRows;
         const long long cost = (tiles + slots - 1) / slots * (rows + 2);
         if (best_cost < 0 || cost < best_cost) {

@@ -621,8 +621,8 @@ __device__ __forceinline__ void segment_tile(const MixedArgs& A, const TileGeom&
     }
 }
 
-// Persistent x sweep: warp w of the W warps of the grid walks the tiles w,
-// w + W, w + 2W, ... of the launch's tile list.  Bounded to 64 (Euler) and 96
+// x sweep: warp w of the W warps of the grid walks the tiles w, w + W,
+// w + 2W, ... of the launch's tile list (launched with a warp per tile).  Bounded to 64 (Euler) and 96
 // (Allaire) registers for 8 and 5 CTAs per SM.
 //
 // Both sweeps are bound by instruction issue: at 2048^2 Euler the x sweep runs

@@ -109,3 +109,29 @@ def test_strands_of_one_form_equal_each_member_alone(recipe, prec, ticks):
         assert (st.t, st.maxu, st.maxv) == (st1.t, st1.maxu, st1.maxv)
         assert np.array_equal(grid, alone)
         assert abs(st.mass1 - st1.mass1) <= 1e-12 * abs(st1.mass1)
+
+
+@pytest.mark.parametrize("prec", [G.MIXED, G.FP64_FAST], ids=["mixed", "fast"])
+@pytest.mark.parametrize("recipe", ["shock_bubbles", "water_shock_air_bubble"])
+def test_many_x_tiles_of_twenty_rows(recipe, prec):
+    """Beside a grid of many tiles a small one's segments have 20 rows, alone
+    others; its bits are the same."""
+    small = G.recipe_config(recipe, 333, 217)
+    large = G.recipe_config(recipe, 2400, 2400)
+    small.precision = large.precision = prec
+    states, rows = [], []
+    for beside in (False, True):
+        with G.Batch() as b:
+            m = b.add_recipe(small, recipe, max_steps=4)
+            if beside:
+                b.add_recipe(large, recipe, max_steps=4)
+            b.step(4)
+            st = b.status(m)
+            states.append((st.n, st.t, st.maxu, st.maxv, b.download(m).tobytes()))
+        with G.Batch() as b:
+            b.add_recipe(small, recipe, max_steps=4)
+            if beside:
+                b.add_recipe(large, recipe, max_steps=4)
+            rows.append(b.segment_rows(small.model, prec))
+    assert rows[1] == 20 and rows[0] != 20
+    assert states[0] == states[1]
