@@ -414,7 +414,9 @@ __device__ __forceinline__ bool hllc_rn(const Eos& q, int wavespeed, const Side<
     const double fac = quot_rn(d, g, rcp_rn(g));
     double pd = quot_rn(p, d, rcp_rn(d));
     pd = left ? -pd : pd;  // p / (S - u)
-    const double wave = left ? smin(0.0, SL) : smax(0.0, SR);
+    // min(0, S_L) or max(0, S_R)
+    const double S = left ? SL : SR;
+    const double wave = (left ? SL : -SR) < 0.0 ? S : 0.0;
     double Us[NV];
 #pragma unroll
     for (int k = 0; k < NV; ++k) Us[k] = fac * U[k];

@@ -465,7 +465,13 @@ __device__ __forceinline__ void copy8_async(double* dst, const double* src) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(src) : "memory");
 }
 
-template <int MODEL, int DIR>
+// A sweep kernel's options: those of its arguments, or MUSCL with one limiter
+// and one wave-speed estimate at compile time (the same operations: the bits
+// do not depend on it).
+constexpr int kAnyOption = -1;
+constexpr int sweep_option(int limiter, int wavespeed) { return 2 * limiter + wavespeed; }
+
+template <int MODEL, int DIR, int OPT>
 __global__ void __launch_bounds__(sweep_threads<DIR>(), sweep_min_ctas<MODEL, DIR>())
     sweep_kernel(SweepArgs A) {
     using MT = ModelTraits<MODEL>;
@@ -519,7 +525,9 @@ __global__ void __launch_bounds__(sweep_threads<DIR>(), sweep_min_ctas<MODEL, DI
         asm volatile("cp.async.commit_group;\n" ::: "memory");
     };
 
-    const SegPar par{A.eos, A.limiter, A.wavespeed, A.godunov, A.z_min};
+    const SegPar par{A.eos, OPT == kAnyOption ? A.limiter : OPT / 2,
+                     OPT == kAnyOption ? A.wavespeed : OPT % 2, OPT == kAnyOption ? A.godunov : 0,
+                     A.z_min};
 
     double r_mu = 0.0, r_mv = 0.0, r_m1 = 0.0, r_m2 = 0.0;
     // this tile and the next (tx across the grid, ty up), stepped by the grid

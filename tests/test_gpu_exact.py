@@ -82,3 +82,25 @@ def test_segment_edges_match_oracle(nx, ny, strang):
         out = s.download()
     assert (st.n, st.t) == (n, t)
     assert np.array_equal(out[2:-2, 2:-2], ref[2:-2, 2:-2])
+
+
+@pytest.mark.parametrize("strang", [0, 1])
+@pytest.mark.parametrize("ws", ["davis", "pvrs"])
+@pytest.mark.parametrize("limiter", ["minmod", "vanleer", "mc", "unlimited"])
+@pytest.mark.parametrize("case", ["shocked_helium_bubble", "underwater_explosion_modified"])
+def test_two_material_options_match_oracle(case, limiter, ws, strang):
+    """The sweeps compiled for a limiter and a wave-speed estimate, and the
+    general ones."""
+    cfg = G.case_config(G.ALLAIRE, case, 45, 31)
+    cfg.limiter, cfg.wavespeed, cfg.splitting = G.LIMITERS[limiter], G.WAVESPEED[ws], strang
+    ic = G.case_ic(cfg, case)
+    p, model = params_from_config(cfg)
+    ref = ic.copy()
+    taken, n, t, _ = O.port_run(model, p, ref, 12)
+    with G.Solver(cfg) as s:
+        s.upload(ic)
+        s.advance(12)
+        st = s.status()
+        out = s.download()
+    assert (st.n, st.t) == (n, t)
+    assert np.array_equal(out[2:-2, 2:-2], ref[2:-2, 2:-2], equal_nan=True)
