@@ -186,6 +186,7 @@ struct cfd_server {
     int64_t completed = 0, rounds = 0, admitted = 0;
     int max_running = 0;
     int worker_error = 0;
+    int copying = 0;  // results being copied out without the lock
     int device = 0;
 };
 
@@ -587,9 +588,11 @@ int cfd_server_wait(cfd_server* s, int64_t id, double timeout_s, cfd_request_inf
     if (result && !failed) {
         // the worker needs the lock between its rounds: copied without it,
         // while `r` keeps the grid from a release on another thread
+        ++s->copying;  // cfd_server_destroy waits for it
         lk.unlock();
         copy_grid(result, r->grid, r->elems);
         lk.lock();
+        if (--s->copying == 0) s->cv_done.notify_all();
     }
     return failed ? cfd_fail(error, "request %lld failed", (long long)id) : CFD_OK;
     // `r` goes before the lock does: the last owner gives the grid back under it
@@ -633,6 +636,10 @@ int cfd_server_destroy(cfd_server* s) {
     }
     s->cv_work.notify_all();
     if (s->worker.joinable()) s->worker.join();
+    {
+        std::unique_lock<std::mutex> lk(s->mu);
+        s->cv_done.wait(lk, [&] { return s->copying == 0; });
+    }
     for (auto& kv : s->reqs) {
         Request* r = kv.second.get();
         if (r->solver) cfd_destroy(r->solver);
