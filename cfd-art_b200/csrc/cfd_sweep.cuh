@@ -24,13 +24,13 @@
 // cfd_exact.cuh, with the plain functions for a segment any lane of which
 // they do not serve.
 //
-// What bounds it: FP64 work.  At 2048^2 Euler the x sweep runs 870 thread
+// What bounds it: FP64 work.  At 2048^2 Euler the x sweep runs 858 thread
 // instructions per cell, 360 of them on the FP64 pipe (53 % busy, 64 % of the
 // issue slots), against 1921 and 478 when every division was made on its own
 // and the phases met in shared memory: x 314 -> 165 us, y 426 -> 194 us.
-// 4096^2 Euler 2.79 -> 1.41 ms a step, Allaire 2048x1024 0.90 -> 0.36 ms, the
-// 200x200 grid 22.0 -> 18.0 us a step, where a launch is one pass through the
-// code.
+// 4096^2 Euler 2.79 -> 1.34 ms a step, Allaire 2048x1024 0.90 -> 0.36 ms (0.33 with
+// its options at compile time), the 200x200 grid 22.0 -> 18.0 us a step, where
+// a launch is one pass through the code.
 #pragma once
 
 #include "cfd_exact.cuh"
