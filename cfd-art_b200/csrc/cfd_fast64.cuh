@@ -644,7 +644,8 @@ __device__ __forceinline__ void march64_strip(const MixedArgs& A, const TileGeom
     bool dummy;
 #pragma unroll
     for (int j = 0; j < kAhead; ++j) {
-        if (r0 - 2 + j <= r1 + 1) stage_issue<MODEL>(stg, j, pin, src_row(r0 - 2 + j, dummy) * pitch + c);
+        if (r0 < r1)  // a part without rows copies none: nothing below would wait for them
+            stage_issue<MODEL>(stg, j, pin, src_row(r0 - 2 + j, dummy) * pitch + c);
         mixed::cp_async_commit();
     }
     int slot = 0;

@@ -293,7 +293,7 @@ __device__ __forceinline__ void march_strip(const MixedArgs& A, const TileGeom& 
     bool ng;
 #pragma unroll
     for (int j = 0; j < kMAhead; ++j) {
-        if (r0 - 2 + j <= r1 + 1)
+        if (r0 < r1)  // a part without rows copies none: nothing below would wait for them
             mstage_issue<MODEL>(stg + j * SB, qin(), (unsigned)src_row(r0 - 2 + j, ng) * pitch + c);
         cp_async_commit();
     }
