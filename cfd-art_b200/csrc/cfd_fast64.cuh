@@ -7,7 +7,7 @@
 // E/headers/flux_solver_MUSCLhancock.hpp:128-227,
 // E/headers/riemann_solver_HLLC.hpp:50-145 and their A/ counterparts),
 // computed for throughput instead of bit identity:
-//   * multiply-adds contracted into FMAs;
+//   * multiply-adds as FMAs, each written as one (see below);
 //   * reciprocals and square roots from the hardware approximations
 //     (PTX rcp.approx.ftz.f64, rsqrt.approx.ftz.f64) refined by one
 //     Newton-Raphson / Householder step to about one ulp, and one reciprocal
@@ -20,6 +20,11 @@
 //     snapping of near-zero partial densities and near-0/1 volume fractions
 //     (A/headers/misc.hpp:251-266) and then the same tests;
 //   * the conservative update applied face by face as the fluxes arrive.
+// No sum here has a plain product for an operand: it is an fma, or the product
+// is a mul().  The compiler may otherwise contract the two in one copy of the
+// code and not in another, and the copies (a loop unrolled by two, each set of
+// options) would give different bits: a strip's rows fall to the one or the
+// other copy by the strip's length, which a member's company in the batch sets.
 // It agrees with the reference to a relative L1 density error far below the
 // 1e-12 bound of the plain form over the benchmarked runs (measured by the
 // tests against the bit-identical form), not bit for bit.
@@ -45,6 +50,9 @@ namespace fast {
 using mixed::Inst;
 using mixed::MixedArgs;
 using mixed::TileGeom;
+
+// A product that is not contracted into the sums it feeds.
+__device__ __forceinline__ double mul(double a, double b) { return __dmul_rn(a, b); }
 
 // Per-tile FP64 constants held in registers.
 struct DPar {
@@ -99,10 +107,8 @@ __device__ __forceinline__ double rsqrt_f(double a) {
     return fma(y * fma(0.375, e, 0.5), e, y);
 }
 // sqrt(a), and sqrt(a / b) = a / sqrt(a b) without the division; 0 for a = 0.
-// (The products are not to be contracted into what follows, so that every
-// instantiation of a sweep gives the same bits.)
-__device__ __forceinline__ double sqrt_f(double a) { return __dmul_rn(a, rsqrt_f(a)); }
-__device__ __forceinline__ double sqrt_ratio(double a, double b) { return __dmul_rn(a, rsqrt_f(a * b)); }
+__device__ __forceinline__ double sqrt_f(double a) { return mul(a, rsqrt_f(a)); }
+__device__ __forceinline__ double sqrt_ratio(double a, double b) { return mul(a, rsqrt_f(mul(a, b))); }
 
 __device__ __forceinline__ int hi32(double x) { return __double2hiint(x); }
 constexpr unsigned kInfHi = 0x7ff00000u;   // high word of infinity
@@ -134,15 +140,15 @@ template <int MODEL>
 __device__ __forceinline__ void c2p(const DPar& P, const double* U, Prim64<MODEL>& Q) {
     if constexpr (MODEL == MODEL_EULER) {
         Q.r = rcp(U[0]);
-        const double u = U[1] * Q.r, v = U[2] * Q.r;
+        const double u = mul(U[1], Q.r), v = mul(U[2], Q.r);
         const double re = fma(-0.5, fma(U[1], u, U[2] * v), U[3]);  // rho e
         Q.W[0] = U[0];
         Q.W[1] = u;
         Q.W[2] = v;
-        Q.W[3] = P.stiff() ? fma(P.gm1, re, -P.gp1) : P.gm1 * re;
+        Q.W[3] = P.stiff() ? fma(P.gm1, re, -P.gp1) : mul(P.gm1, re);
     } else {
         Q.r = rcp(U[0] + U[1]);
-        const double u = U[2] * Q.r, v = U[3] * Q.r;
+        const double u = mul(U[2], Q.r), v = mul(U[3], Q.r);
         const double re = fma(-0.5, fma(U[2], u, U[3] * v), U[4]);
         double eps;
         mix_eps_kn<MODEL>(P, U[5], eps, Q.kn);
@@ -151,7 +157,7 @@ __device__ __forceinline__ void c2p(const DPar& P, const double* U, Prim64<MODEL
         Q.W[1] = U[1];
         Q.W[2] = u;
         Q.W[3] = v;
-        Q.W[4] = (re - Q.kn) * Q.ie;
+        Q.W[4] = mul(re - Q.kn, Q.ie);
         Q.W[5] = U[5];
     }
 }
@@ -249,31 +255,34 @@ __device__ __forceinline__ void hi_range(int q, const double* a, const double* b
 template <int MODEL>
 __device__ __forceinline__ void face_states(const DPar& P, const Prim64<MODEL>& Q, const double* d,
                                             double s, double* Wp, double* Wm, bool& okp, bool& okm) {
-    constexpr int NV = ModelTraits<MODEL>::NV;
+    using T = ModelTraits<MODEL>;
+    constexpr int NV = T::NV;
     const double* W = Q.W;
     double E[NV], D[NV], X[NV];
     const double rc2 = rho_c2<MODEL>(P, W, Q.ie, Q.kn);
+    const double su = s * W[T::IM];
     if constexpr (MODEL == MODEL_EULER) {
-        const double su = s * W[1];
         X[0] = fma(su, d[0], (s * W[0]) * d[1]);
         X[1] = fma(su, d[1], (s * Q.r) * d[3]);
-        X[2] = su * d[2];
         X[3] = fma(su, d[3], (s * rc2) * d[1]);
     } else {
-        const double su = s * W[2], sd = s * d[2];
+        const double sd = s * d[2];
         X[0] = fma(su, d[0], W[0] * sd);
         X[1] = fma(su, d[1], W[1] * sd);
         X[2] = fma(su, d[2], (s * Q.r) * d[4]);
-        X[3] = su * d[3];
         X[4] = fma(su, d[4], rc2 * sd);
-        X[5] = su * d[5];
     }
 #pragma unroll
     for (int q = 0; q < NV; ++q) {
         E[q] = fma(0.5, d[q], W[q]);
         D[q] = fma(-0.5, d[q], W[q]);
-        Wp[q] = E[q] - X[q];
-        Wm[q] = D[q] - X[q];
+        if (q == T::IT || q == 5) {  // X = su d alone
+            Wp[q] = fma(-su, d[q], E[q]);
+            Wm[q] = fma(-su, d[q], D[q]);
+        } else {
+            Wp[q] = E[q] - X[q];
+            Wm[q] = D[q] - X[q];
+        }
     }
     bool ok;
     unsigned lo, up, lop, upp;
@@ -309,7 +318,7 @@ __device__ __forceinline__ void face_states(const DPar& P, const Prim64<MODEL>& 
 template <int MODEL>
 __device__ __forceinline__ double sound(const DPar& P, const double* W, double r, double ie,
                                         double kn) {
-    return sqrt_f(rho_c2<MODEL>(P, W, ie, kn) * r);
+    return sqrt_f(mul(rho_c2<MODEL>(P, W, ie, kn), r));
 }
 
 // HLLC flux from primitive face states (E/headers/riemann_solver_HLLC.hpp:50-145,
@@ -356,11 +365,11 @@ __device__ __forceinline__ void hllc(const DPar& P, const double* WL, const doub
         SL = uL - (ppv > pL ? sqrt_ratio(fma(ppv, eL, fma(0.5, ppv + pL, knL)), MLe) : cL);
         SR = uR + (ppv > pR ? sqrt_ratio(fma(ppv, eR, fma(0.5, ppv + pR, knR)), MRe) : cR);
     } else {
-        const double ua = 0.5 * (uL + uR), ca = 0.5 * (cL + cR);
-        SL = dmin(ua - ca, uL - cL);
-        SR = dmax(ua + ca, uR + cR);
+        const double us = uL + uR, ca = 0.5 * (cL + cR);
+        SL = dmin(fma(0.5, us, -ca), uL - cL);
+        SR = dmax(fma(0.5, us, ca), uR + cR);
     }
-    const double mL = rhoL * (SL - uL), mR = rhoR * (SR - uR);
+    const double mL = mul(rhoL, SL - uL), mR = mul(rhoR, SR - uR);
     // u* = num/den; its sign, and 1/(S - u*) = den/(S den - num), do not wait
     // for the quotient
     const double num = fma(-mR, uR, fma(mL, uL, pR - pL)), den = mL - mR;
@@ -370,8 +379,8 @@ __device__ __forceinline__ void hllc(const DPar& P, const double* WL, const doub
     const double v = left ? WL[T::IT] : WR[T::IT];
     const double Sk = left ? SL : SR, wave = left ? dmin(0.0, SL) : dmax(0.0, SR);
     const double q = den * rcp(fma(Sk, den, -num));  // 1/(S - u*)
-    const double u_star = num * rcp(den);
-    const double fac = (Sk - u) * q;    // (S - u)/(S - u*)
+    const double u_star = mul(num, rcp(den));
+    const double fac = mul(Sk - u, q);  // (S - u)/(S - u*)
     // The passive components' flux U u + w (fac U - U) is U A; the normal
     // momentum's rho (u^2 + w (fac u* - u)) + p; the energy's star state
     // fac (E + (u* - u)(rho u* + p/(S - u))) - E gives E A + p u
@@ -385,17 +394,17 @@ __device__ __forceinline__ void hllc(const DPar& P, const double* WL, const doub
         re = fma(p, eps, kn);  // (p + k) eps
     }
     const double E = fma(0.5 * rho, fma(u, u, v * v), re);
-    const double m = rho * A, fu = fac * u_star;
+    const double m = mul(rho, A), fu = mul(fac, u_star);
     if constexpr (MODEL == MODEL_EULER) {
         F[0] = m;
     } else {
-        F[0] = (left ? WL[0] : WR[0]) * A;
-        F[1] = (left ? WL[1] : WR[1]) * A;
+        F[0] = mul(left ? WL[0] : WR[0], A);
+        F[1] = mul(left ? WL[1] : WR[1], A);
         F[5] = 0.0;
         F[NV + 1] = left ? WL[5] : WR[5];
     }
     F[T::IM] = fma(rho, fma(wave, fu - u, u * u), p);
-    F[T::IT] = m * v;
+    F[T::IT] = mul(m, v);
     F[T::IE] = fma(wave * (u_star - u), fma(rho, fu, p * q), fma(E, A, p * u));
     F[NV] = u_star;
 }
@@ -407,9 +416,9 @@ __device__ __forceinline__ double z_new(bool god, double k, double zL, double z,
                                         double z_min) {
     double nz;
     if (god)
-        nz = z - k * fma(zR - z, dmin(0.0, usR), (z - zL) * dmax(0.0, usL));
+        nz = fma(-k, fma(zR - z, dmin(0.0, usR), (z - zL) * dmax(0.0, usL)), z);
     else
-        nz = z - k * (fma(usR, zsR, -usL * zsL) - z * (usR - usL));
+        nz = fma(-k, fma(-z, usR - usL, fma(usR, zsR, -usL * zsL)), z);
     const double lo = z_min > 0.0 ? z_min : 0.0, hi = z_min > 0.0 ? 1.0 - z_min : 1.0;
     return dmax(dmin(hi, nz), lo);
 }
@@ -439,17 +448,17 @@ __device__ __forceinline__ void repair(double* N, const double* Uold) {
         if (euler_physical(N)) return;
         double rho = N[0];
         const double u = N[1] / rho, v = N[2] / rho;
-        double e = N[3] / rho - 0.5 * (u * u + v * v);
+        double e = fma(-0.5, fma(u, u, v * v), N[3] / rho);
         const double ro = Uold[0];
         const double uo = Uold[1] / ro, vo = Uold[2] / ro;
-        const double eo = Uold[3] / ro - 0.5 * (uo * uo + vo * vo);
+        const double eo = fma(-0.5, fma(uo, uo, vo * vo), Uold[3] / ro);
         if (rho <= 1e-12) rho = ro;
         if (e <= 1e-12) e = eo;
         // the pressure of (e, rho) taken back to conserved: rho e + rho |u|^2 / 2
         N[0] = rho;
         N[1] = rho * u;
         N[2] = rho * v;
-        N[3] = rho * e + 0.5 * rho * (u * u + v * v);
+        N[3] = fma(0.5 * rho, fma(u, u, v * v), rho * e);
     }
 }
 

@@ -94,7 +94,7 @@ __device__ __forceinline__ void block_count(unsigned long long* ctr, int idx, bo
 __device__ __forceinline__ double choose_dt(const DevState& s, double maxu, double maxv) {
     double cfl = s.cfl;
     if (s.n < 5) cfl = smin(cfl, 0.2);
-    double dt = cfl * smin(s.dx / maxu, s.dy / maxv);
+    double dt = __dmul_rn(cfl, smin(s.dx / maxu, s.dy / maxv));  // not contracted into the sum
     if (s.t + dt > s.T) dt = s.T - s.t;
     return dt;
 }

@@ -28,7 +28,7 @@ def _run(cfg, recipe, copies=1, rows=0):
 
 @pytest.mark.parametrize("recipe,prec", [("water_shock_air_bubble", G.FP64_FAST),
                                          ("water_shock_air_bubble", G.MIXED),
-                                         ("shock_bubbles", G.MIXED)])
+                                         ("shock_bubbles", G.FP64_FAST), ("shock_bubbles", G.MIXED)])
 @pytest.mark.parametrize("nx,ny", [(700, 500), (640, 612), (900, 900), (64, 65), (200, 49)])
 def test_parts_without_rows(recipe, prec, nx, ny):
     cfg = G.recipe_config(recipe, nx, ny)
