@@ -181,6 +181,7 @@ def lib() -> C.CDLL:
             "cfd_batch_set_march_rows": (ip, [vp, ip, ip]),
             "cfd_batch_get_march_rows": (ip, [vp, ip, C.POINTER(ip)]),
             "cfd_batch_get_segment_rows": (ip, [vp, ip, ip, C.POINTER(ip)]),
+            "cfd_batch_get_split": (ip, [vp, ip, ip, C.POINTER(ip), C.POINTER(ip)]),
             "cfd_batch_status": (ip, [vp, ip, C.POINTER(Status)]),
             "cfd_batch_poll_issue": (ip, [vp]),
             "cfd_batch_poll_collect": (ip, [vp, ip, C.POINTER(ip), C.POINTER(ip), C.POINTER(ip), dp,
@@ -517,6 +518,13 @@ class Batch:
         check(lib().cfd_batch_get_segment_rows(self._h, model, precision, C.byref(r)),
               "cfd_batch_get_segment_rows")
         return r.value
+
+    def split(self, model: int, precision: int = MIXED) -> tuple[int, int]:
+        """Parts that the tiles of the x and y sweeps are divided into."""
+        x, y = C.c_int(), C.c_int()
+        check(lib().cfd_batch_get_split(self._h, model, precision, C.byref(x), C.byref(y)),
+              "cfd_batch_get_split")
+        return x.value, y.value
 
     def status(self, mid: int) -> Status:
         st = Status()

@@ -314,6 +314,11 @@ int cfd_batch_get_march_rows(cfd_batch* b, int model, int* rows);
  * tiles fill the resident warps; 0 when that model and form have no active
  * member.  Results do not depend on it. */
 int cfd_batch_get_segment_rows(cfd_batch* b, int model, int precision, int* rows);
+/* Parts that the tiles of the x and y sweeps of a model and form are divided
+ * into in the current tile list (the largest, where its members step in
+ * several strands): 1 undivided, 0 when that model and form have no active
+ * member.  Results do not depend on it. */
+int cfd_batch_get_split(cfd_batch* b, int model, int precision, int* x, int* y);
 int cfd_batch_status(cfd_batch* b, int id, cfd_status* st);
 /* ids, steps taken, done flags and times of all members (cap entries). */
 int cfd_batch_poll(cfd_batch* b, int cap, int* ids, int* steps, int* done, double* t, int* count);
