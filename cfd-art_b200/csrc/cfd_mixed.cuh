@@ -135,12 +135,13 @@ __device__ __forceinline__ float frcp(float x) { return 1.0f / x; }
 // a wave speed or a product of them, is many orders of magnitude smaller).
 // Measured 3-4 % faster on the sweeps, the same results on every test case.
 __device__ __forceinline__ float fdiv(float a, float b) { return __fdividef(a, b); }
-// sqrt(a / b) for b > 0 as a / sqrt(a b), with a at least 1e-30 (a root of
-// 1e-15 where it is 0 or negative): two instructions beside the hardware's.
-__device__ __forceinline__ float sqrt_ratio(float a, float b) {
-    const float x = fmaxf(a, 1e-30f);
-    return __fmul_rn(x, rsqrtf(x * b));
-}
+// sqrt(a / b) for b > 0: the root of the quotient, so that a and b may each take
+// FP32's range.  (a rsqrt(a b) is 0 or infinite where the product leaves it; it
+// takes 99.0 us a tick of Euler 2048^2 and 96.3 of Allaire 2048x1024, this 99.2
+// and 96.9, and that form with a test of its result 98.7 to 100.0 and 101.8 to
+// 103.7.)  At least 3e-19, where a is 0 or negative too: a gas of no pressure at
+// rest keeps S_L < S_R.
+__device__ __forceinline__ float sqrt_ratio(float a, float b) { return sqrtf(fmaxf(1e-37f, fdiv(a, b))); }
 // One instruction each (the comparison forms of the reference's std::min and
 // std::max take two); a NaN operand gives the other one.
 __device__ __forceinline__ float fminf_s(float a, float b) { return fminf(a, b); }
