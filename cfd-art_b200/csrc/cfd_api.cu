@@ -85,9 +85,11 @@ namespace {
 #define CUDA_TRY(expr)                                                                   \
     do {                                                                                 \
         cudaError_t e_ = (expr);                                                         \
-        if (e_ != cudaSuccess)                                                           \
+        if (e_ != cudaSuccess) {                                                         \
+            cudaGetLastError(); /* not left to the next launch's check */                \
             return fail(e_ == cudaErrorMemoryAllocation ? CFD_ERR_NOMEM : CFD_ERR_CUDA,  \
                         "%s: %s (%s:%d)", #expr, cudaGetErrorString(e_), __FILE__, __LINE__); \
+        }                                                                                \
     } while (0)
 
 constexpr int kSMs = 148;
@@ -852,11 +854,13 @@ int cfd_upload(cfd_solver* s, const double* host, int layout, int n, double t) {
     int r;
     if (layout != CFD_LAYOUT_GHOSTED_AOS && layout != CFD_LAYOUT_SOA)
         return fail(CFD_ERR_INVALID, "unknown layout %d", layout);
-    if ((r = set_time(s, n, t))) return r;
+    // the time is set only once the copy is queued: one that is refused leaves
+    // the solver at its state and time
     if (layout == CFD_LAYOUT_GHOSTED_AOS) {
         size_t elems = (size_t)s->nv * (c.nx + 2 * s->g) * (size_t)(c.ny + 2 * s->g);
         CUDA_TRY(cudaMemcpyAsync(s->buf[1], host, elems * sizeof(double), cudaMemcpyHostToDevice,
                                  s->stream));
+        if ((r = set_time(s, n, t))) return r;
         if ((r = enqueue_load<kFromAos>(s, s->buf[1]))) return r;
         if (s->frame) {
             frame_from_ghosted<<<148, 256, 0, s->stream>>>(s->buf[1], s->frame, c.nx, c.ny, s->g,
@@ -869,6 +873,7 @@ int cfd_upload(cfd_solver* s, const double* host, int layout, int n, double t) {
                                        host + (size_t)k * c.nx * c.ny, c.nx * sizeof(double),
                                        c.nx * sizeof(double), c.ny, cudaMemcpyHostToDevice,
                                        s->stream));
+        if ((r = set_time(s, n, t))) return r;
         if (s->frame && (r = frame_from_state(s))) return r;
         if ((r = enqueue_load<kInPlace>(s, nullptr))) return r;
     }
@@ -880,7 +885,6 @@ int cfd_upload_device(cfd_solver* s, const double* dev, int n, double t) {
     if (!s || !dev) return fail(CFD_ERR_INVALID, "null argument");
     const cfd_config& c = s->cfg;
     int r;
-    if ((r = set_time(s, n, t))) return r;
     // this device's own memory is read by the kernel, anything else that
     // a copy takes (another device's memory, the host's, unaligned or the
     // solver's own planes) is copied
@@ -895,6 +899,7 @@ int cfd_upload_device(cfd_solver* s, const double* dev, int n, double t) {
                       (a + bytes <= own || own + sizeof(double) * s->nv * s->plane <= a);
     cudaGetLastError();
     if (here) {
+        if ((r = set_time(s, n, t))) return r;
         if ((r = enqueue_load<kFromPlanes>(s, dev))) return r;
     } else {
         for (int k = 0; k < s->nv; ++k)
@@ -902,6 +907,7 @@ int cfd_upload_device(cfd_solver* s, const double* dev, int n, double t) {
                                        dev + (size_t)k * c.nx * c.ny, c.nx * sizeof(double),
                                        c.nx * sizeof(double), c.ny, cudaMemcpyDeviceToDevice,
                                        s->stream));
+        if ((r = set_time(s, n, t))) return r;
         if ((r = enqueue_load<kInPlace>(s, nullptr))) return r;
     }
     if (s->frame && (r = frame_from_state(s))) return r;

@@ -1,0 +1,54 @@
+"""An upload that is refused leaves the solver as it was.  The planes handed over
+are larger than the allocation they lie in, which the driver's copies refuse.
+(The next allocation follows it directly, so the memory past its end exists.)"""
+import ctypes
+
+import numpy as np
+import pytest
+
+import cfdgpu as G
+
+pytestmark = pytest.mark.gpu
+
+FIELDS = ("n", "t", "dt_next", "maxu", "maxv", "mass1", "mass2")
+
+
+def _adjacent(driver, size):
+    """Device allocations of `size` bytes, and one of them whose end another begins at."""
+    got = []
+    for _ in range(16):
+        p = ctypes.c_uint64()
+        assert driver.cuMemAlloc_v2(ctypes.byref(p), ctypes.c_size_t(size)) == 0
+        got.append(p.value)
+    return got, next((p for p in got if p + size in got), None)
+
+
+@pytest.mark.parametrize("steps", [1, 2])
+@pytest.mark.parametrize("offset", [4], ids=["copied"])
+def test_refused_upload_changes_nothing(offset, steps):
+    cfg = G.recipe_config("shock_bubbles", 64, 64)
+    cfg.splitting = 1  # an odd number of sweeps a step: the current buffer alternates
+    ic = G.recipe_ic(cfg, "shock_bubbles", nbubbles=4)
+    driver = ctypes.CDLL("libcuda.so.1")
+    with G.Solver(cfg) as s, G.Solver(cfg) as untouched:
+        for x in (s, untouched):
+            x.upload(ic)
+            x.advance(steps)
+        before = [getattr(s.status(), f) for f in FIELDS]
+        state = s.download()
+        size = 64 * 64 * 8 * 3 // 2  # a plane and a half of four
+        all_, small = _adjacent(driver, size)
+        try:
+            if small is None:
+                pytest.skip("no two adjacent allocations")
+            with pytest.raises(G.CfdError):
+                s.upload_device(small + offset, n=70, t=0.5)
+        finally:
+            for p in all_:
+                driver.cuMemFree_v2(ctypes.c_uint64(p))
+        assert [getattr(s.status(), f) for f in FIELDS] == before
+        if steps % 2:  # the copy goes to the other buffer then, as far as it got
+            assert np.array_equal(s.download(), state)
+            s.advance(3)
+            untouched.advance(3)
+            assert np.array_equal(s.download(), untouched.download())
