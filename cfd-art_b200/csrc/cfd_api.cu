@@ -1,6 +1,7 @@
 // C ABI of the B200 split finite-volume solver: solver objects, device
 // memory, layout conversion and launch of the sweep kernels.  Compiled with
 // --fmad=false (see __graft_entry__.build) like the kernels it instantiates.
+#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -881,24 +882,43 @@ int cfd_upload(cfd_solver* s, const double* host, int layout, int n, double t) {
     return CFD_OK;
 }
 
+// Whether `bytes` from `p` on are this device's own memory, of one allocation.
+// Memory mapped in pieces counts as one allocation a piece.
+static bool own_range(const void* p, size_t bytes) {
+    using Range = CUresult (*)(CUdeviceptr*, size_t*, CUdeviceptr);
+    static const Range range = [] {
+        void* f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &f, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess)
+            f = nullptr;
+        cudaGetLastError();
+        return reinterpret_cast<Range>(f);
+    }();
+    cudaPointerAttributes pa = {};
+    int device = -1;
+    const bool here = cudaGetDevice(&device) == cudaSuccess &&
+                      cudaPointerGetAttributes(&pa, p) == cudaSuccess &&
+                      pa.type == cudaMemoryTypeDevice && pa.device == device;
+    cudaGetLastError();
+    CUdeviceptr base = 0;
+    size_t size = 0;
+    const CUdeviceptr a = (CUdeviceptr)(uintptr_t)p;
+    return here && range && range(&base, &size, a) == CUDA_SUCCESS && a + bytes <= base + size;
+}
+
 int cfd_upload_device(cfd_solver* s, const double* dev, int n, double t) {
     if (!s || !dev) return fail(CFD_ERR_INVALID, "null argument");
     const cfd_config& c = s->cfg;
     int r;
-    // this device's own memory is read by the kernel, anything else that
-    // a copy takes (another device's memory, the host's, unaligned or the
-    // solver's own planes) is copied
+    // planes within an allocation of this device are read by the kernel, anything
+    // else that a copy takes (another device's memory, the host's, unaligned or the
+    // solver's own planes) is copied, and what a copy refuses (planes that go
+    // past their allocation) is refused by it
     const size_t bytes = sizeof(double) * s->nv * c.nx * (size_t)c.ny;
     const uintptr_t a = (uintptr_t)dev, own = (uintptr_t)s->buf[0];
-    cudaPointerAttributes pa = {};
-    int device = -1;
-    const bool here = cudaGetDevice(&device) == cudaSuccess &&
-                      cudaPointerGetAttributes(&pa, dev) == cudaSuccess &&
-                      pa.type == cudaMemoryTypeDevice && pa.device == device &&
-                      a % sizeof(double) == 0 &&
-                      (a + bytes <= own || own + sizeof(double) * s->nv * s->plane <= a);
-    cudaGetLastError();
-    if (here) {
+    if (a % sizeof(double) == 0 && own_range(dev, bytes) &&
+        (a + bytes <= own || own + sizeof(double) * s->nv * s->plane <= a)) {
         if ((r = set_time(s, n, t))) return r;
         if ((r = enqueue_load<kFromPlanes>(s, dev))) return r;
     } else {

@@ -24,7 +24,7 @@ def _adjacent(driver, size):
 
 
 @pytest.mark.parametrize("steps", [1, 2])
-@pytest.mark.parametrize("offset", [4], ids=["copied"])
+@pytest.mark.parametrize("offset", [4, 0], ids=["copied", "aligned"])
 def test_refused_upload_changes_nothing(offset, steps):
     cfg = G.recipe_config("shock_bubbles", 64, 64)
     cfg.splitting = 1  # an odd number of sweeps a step: the current buffer alternates
