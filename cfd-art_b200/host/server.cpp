@@ -29,6 +29,7 @@
 
 #include "../../include/cfdgpu.h"
 #include "../../include/cfdgpu_host.h"
+#include "../csrc/cfd_copy.h"
 #include "../csrc/cfd_error.h"
 
 namespace {
@@ -55,18 +56,17 @@ void copy_grid(double* dst, const double* src, size_t elems) {
         memcpy(dst, src, bytes);
         return;
     }
-    const size_t step = (bytes / parts + 4095) / 4096 * 4096;
     std::thread pool[kCopyThreads];
     for (size_t k = 1; k < parts; ++k) {
-        const size_t lo = k * step, n = std::min(step, bytes - lo);
-        auto part = [=] { memcpy((char*)dst + lo, (const char*)src + lo, n); };
+        const cfd::CopyPart p = cfd::copy_part(bytes, parts, k);
+        auto part = [=] { memcpy((char*)dst + p.lo, (const char*)src + p.lo, p.n); };
         try {
             pool[k] = std::thread(part);
         } catch (...) {  // no thread, or no memory for one
             part();
         }
     }
-    memcpy(dst, src, step);
+    memcpy(dst, src, cfd::copy_part(bytes, parts, 0).n);
     for (size_t k = 1; k < parts; ++k)
         if (pool[k].joinable()) pool[k].join();
 }
