@@ -514,7 +514,7 @@ struct cfd_batch {
     // graph of `graph_steps` ticks for the current membership
     cudaGraphExec_t graph = nullptr;
     int graph_steps = 0;
-    int table_ticks = 0;  // ticks run since the tile lists were built
+    long long table_ticks = 0;  // ticks run since the tile lists were built
     // autotuning state
     bool tuned = false;
     int tune_override = -1;
