@@ -193,12 +193,12 @@ int march_rows(const std::vector<std::pair<int, int>>& grids, long long slots) {
 }
 
 // Row count of the x sweep's warp segments over the given grids: tiles of
-// kSegCells columns, a warp walks ceil(tiles / slots) of them one after the
-// other, each costing its rows plus about two rows' worth of setup (the
+// kSegCells columns, a warp each, ceil(tiles / slots) rounds of resident
+// warps, each costing a tile's rows plus about two rows' worth of setup (the
 // member's constants, the first row's load), so the count with the fewest
 // (rounds x (rows + 2)) is taken, the largest on ties.  A lone grid that
 // leaves resident warps idle at 32 rows gets shorter tiles.  From two rounds
-// of tiles of kManyRows on rounds no longer matter (launch_warp): at 2900^2
+// of tiles of kManyRows on the rounds run into one another (launch_warp): at 2900^2
 // the rule's 28 to 32 rows take 99.4 us (Euler mixed), 132.4 (fast) and 210.3
 // (Allaire fast, 2048^2 115.2), 20 rows 93.2, 132.6 and 212.7 (115.5), 16 rows
 // 91.9, 132.5 and 210.7 (113.3), but Allaire mixed 2048^2 83.4 against 81.3.

@@ -924,14 +924,12 @@ __device__ __forceinline__ void segment64_tile(const MixedArgs& A, const TileGeo
 // instructions in x): x 90.6 -> 63.8 us, y 121.1 -> 87.6, then 85.5 us.
 template <int MODEL, int OPT>
 __global__ void __launch_bounds__(128, MODEL == MODEL_EULER ? 5 : 4) fast_segment_x_kernel(MixedArgs A) {
-    const int gw = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int nw = gridDim.x * (blockDim.x >> 5);
-    for (int w = gw; w < A.ntiles * A.split; w += nw) {
-        const TileGeom g = mixed::tile_geom<DIR_X, mixed::kSegCells, mixed::kSegRows>(A, w / A.split);
-        if (g.skip) continue;
-        const int n = mixed::part_rows(A), r = g.b_org + (w % A.split) * n;  // this warp's rows
-        segment64_tile<MODEL, OPT>(A, g, r, min(r + n, g.b_org + A.rows));
-    }
+    const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (w >= A.ntiles * A.split) return;
+    const TileGeom g = mixed::tile_geom<DIR_X, mixed::kSegCells, mixed::kSegRows>(A, w / A.split);
+    if (g.skip) return;
+    const int n = mixed::part_rows(A), r = g.b_org + (w % A.split) * n;  // this warp's rows
+    segment64_tile<MODEL, OPT>(A, g, r, min(r + n, g.b_org + A.rows));
 }
 
 }  // namespace fast

@@ -621,9 +621,7 @@ __device__ __forceinline__ void segment_tile(const MixedArgs& A, const TileGeom&
     }
 }
 
-// x sweep: warp w of the W warps of the grid walks the tiles w, w + W,
-// w + 2W, ... of the launch's tile list (launched with a warp per tile).
-// Bounded to 64 (Euler) and 96 (Allaire) registers for 8 and 5 CTAs per SM.
+// x sweep: a warp per part of a tile.  Bounded to 64 (Euler) and 96 (Allaire) registers for 8 and 5 CTAs per SM.
 //
 // Both sweeps are bound by instruction issue: at 2048^2 Euler the x sweep runs
 // 263 thread instructions a cell (71 % of the issue slots, 5.3 TB/s of its
@@ -639,14 +637,12 @@ __device__ __forceinline__ void segment_tile(const MixedArgs& A, const TileGeom&
 template <int MODEL, int OPT>
 __global__ void __launch_bounds__(128, MODEL == MODEL_EULER ? 8 : 5)
     mixed_segment_x_kernel(MixedArgs A) {
-    const int gw = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int nw = gridDim.x * (blockDim.x >> 5);
-    for (int w = gw; w < A.ntiles * A.split; w += nw) {
-        const TileGeom g = tile_geom<DIR_X, kSegCells, kSegRows>(A, w / A.split);
-        if (g.skip) continue;
-        const int n = part_rows(A), r = g.b_org + (w % A.split) * n;  // this warp's rows
-        segment_tile<MODEL, OPT>(A, g, r, min(r + n, g.b_org + A.rows));
-    }
+    const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if (w >= A.ntiles * A.split) return;
+    const TileGeom g = tile_geom<DIR_X, kSegCells, kSegRows>(A, w / A.split);
+    if (g.skip) return;
+    const int n = part_rows(A), r = g.b_org + (w % A.split) * n;  // this warp's rows
+    segment_tile<MODEL, OPT>(A, g, r, min(r + n, g.b_org + A.rows));
 }
 
 }  // namespace mixed
