@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdarg>
 #include <cstdio>
@@ -201,7 +202,8 @@ int sweep_blocks(const cfd_config& c) {
 template <int MODEL, int DIR, int OPT>
 int launch_sweep_t(const SweepArgs& a, cudaStream_t st) {
     constexpr int smem = sweep_smem_bytes<MODEL, DIR>();
-    static int per_sm = 0;
+    static std::atomic<int> known{0};  // any thread may launch first
+    int per_sm = known.load(std::memory_order_relaxed);
     if (!per_sm) {
         int n = 0;
         CUDA_TRY(cudaFuncSetAttribute(sweep_kernel<MODEL, DIR, OPT>,
@@ -209,6 +211,7 @@ int launch_sweep_t(const SweepArgs& a, cudaStream_t st) {
         CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, sweep_kernel<MODEL, DIR, OPT>,
                                                                sweep_threads<DIR>(), smem));
         per_sm = std::max(1, std::min(n, kMaxCtas / kSMs));
+        known.store(per_sm, std::memory_order_relaxed);
     }
     const long long tiles = sweep_tiles<DIR>(a.nx, a.ny);
     const int grid = (int)std::min<long long>(tiles, per_sm * kSMs);

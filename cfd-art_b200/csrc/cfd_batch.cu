@@ -19,6 +19,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -73,7 +74,8 @@ constexpr int kMarchShape = 3;
 template <int MODEL, int DIR, int TS, int NA>
 int launch_t(const MixedArgs& a, int sms, cudaStream_t st) {
     constexpr int smem = MTile<MODEL, DIR, TS, NA>::SMEM;
-    static int per_sm = 0;
+    static std::atomic<int> known{0};  // any thread may launch first
+    int per_sm = known.load(std::memory_order_relaxed);
     if (!per_sm) {
         cudaError_t e = cudaFuncSetAttribute(mixed_sweep_kernel<MODEL, DIR, TS, NA>,
                                              cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -81,6 +83,7 @@ int launch_t(const MixedArgs& a, int sms, cudaStream_t st) {
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(
             &per_sm, mixed_sweep_kernel<MODEL, DIR, TS, NA>, 256, smem);
         if (e != cudaSuccess || per_sm < 1) per_sm = 1;
+        known.store(per_sm, std::memory_order_relaxed);
     }
     int grid = std::max(1, std::min(a.ntiles, per_sm * sms));
     MixedArgs b = a;
@@ -129,13 +132,15 @@ WarpKernel warp_kernel(int model, int fp64, int dir, int opt) {
 
 // Resident CTAs per SM of such a kernel.
 int warp_per_sm(int model, int fp64, int dir, int opt) {
-    static int known[2][2][2][MF_OPTIONS + 2] = {};
-    int& n = known[model][fp64][dir][opt + 1];
+    static std::atomic<int> known[2][2][2][MF_OPTIONS + 2] = {};  // any thread may launch first
+    std::atomic<int>& at = known[model][fp64][dir][opt + 1];
+    int n = at.load(std::memory_order_relaxed);
     if (!n) {
         const WarpKernel k = warp_kernel(model, fp64, dir, opt);
         int v = 0;
         const cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&v, k.fn, 128, k.smem);
         n = e != cudaSuccess || v < 1 ? 1 : v;
+        at.store(n, std::memory_order_relaxed);
     }
     return n;
 }

@@ -41,10 +41,10 @@ double secs(Clock::time_point a, Clock::time_point b) {
 }
 
 // Copies a whole grid between the caller's memory and the request's.  One
-// core copies about 10 GB/s, a fifth of what the link to the device takes,
-// and a served mix spends longer in these copies than on the device: a copy is
+// core copies about 9 GB/s, a fifth of what the link to the device takes,
+// and the copies of a served mix keep its requests from the device: a copy is
 // cut among up to kCopyThreads threads in parts of at least kCopyPart bytes (a
-// thread costs about 20 us, 2 MB about 200 us).  A part whose thread cannot be
+// thread costs about 20 us, 2 MB about 120 to 200 us).  A part whose thread cannot be
 // started is copied by the caller.
 constexpr size_t kCopyPart = 2u << 20;
 constexpr size_t kCopyThreads = 8;
