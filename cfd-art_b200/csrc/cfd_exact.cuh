@@ -33,8 +33,12 @@
 // value just below a power of two, which densities near 1 do take).  There
 // it gives the power of two below, and RN(1/b) is the next number up.
 //
-// Square roots: g1 = RN(g + r h) from the refined hardware approximation
-// (PTX rsqrt.approx.ftz.f64), g = RN(a y), h = y/2, r = RN(a - g^2); then
+// Square roots: the hardware approximation of 1/sqrt(a) (PTX
+// rsqrt.approx.ftz.f64) refined by one Householder step of order 3 (A. S.
+// Householder, "The Numerical Treatment of a Single Nonlinear Equation", 1970),
+// y (1 + e/2 + 3 e^2/8) with e = 1 - a y^2, then one Newton step on the root
+// itself, its residual exact by FMA (Markstein, above): g1 = RN(g + r h) with
+// g = RN(a y), h = y/2, r = RN(a - g^2); then
 // c = (a - g1^2) h is sqrt(a) - g1 to a relative 2^-40, and g1 is the correctly
 // rounded root whenever |c| is below half an ulp of g1 by its high word.  It
 // is for all but about one operand in a million; the others take the ordinary

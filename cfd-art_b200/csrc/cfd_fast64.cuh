@@ -913,15 +913,16 @@ __device__ __forceinline__ void segment64_tile(const MixedArgs& A, const TileGeo
 // 5 and 11 % slower.
 //
 // Both sweeps wait on FP64 latency at 16-20 warps per SM, with the FP64 pipe
-// half busy: at 2048^2 Euler the x sweep runs 371 thread instructions a cell,
+// half busy: at 2048^2 Euler the x sweep runs 369 thread instructions a cell,
 // about 155 of them FP64, and the y sweep 384, against 533 and 520 before
 // minmod took seven instructions, the physicality tests were made on high
 // words, first-order faces were left to a vote, HLLC's star state was reduced
 // to one reciprocal that does not wait for u*, sound speeds took one
 // reciprocal root and the options were fixed at compile time: x 96.7 -> 74.5
-// us, y 108.4 -> 90.7 us a sweep (72.3 since a warp takes one tile, 84.4 since
-// close_steps closes the steps).  Allaire at 2048x1024 (880 -> 580
-// instructions in x): x 90.6 -> 63.8 us, y 121.1 -> 87.6, then 85.5 us.
+// us, y 108.4 -> 90.7 us a sweep (71.5 since a warp takes one tile, 84.2 since
+// close_steps closes the steps; 73.0 and 84.5 with every multiply-add written
+// out).  Allaire at 2048x1024 (880 -> 558 instructions in x): x 90.6 -> 63.8 us,
+// y 121.1 -> 87.6, then 84.6 us.
 template <int MODEL, int OPT>
 __global__ void __launch_bounds__(128, MODEL == MODEL_EULER ? 5 : 4) fast_segment_x_kernel(MixedArgs A) {
     const int w = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);

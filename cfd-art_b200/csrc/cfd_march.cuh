@@ -624,14 +624,14 @@ __device__ __forceinline__ void segment_tile(const MixedArgs& A, const TileGeom&
 // x sweep: a warp per part of a tile.  Bounded to 64 (Euler) and 96 (Allaire) registers for 8 and 5 CTAs per SM.
 //
 // Both sweeps are bound by instruction issue: at 2048^2 Euler the x sweep runs
-// 263 thread instructions a cell (71 % of the issue slots, 5.3 TB/s of its
-// 268 MB, 81 % of the measured copy) and the y sweep 266 (68 %, 4.6 TB/s with
+// 263 thread instructions a cell (73 % of the issue slots, 5.3 TB/s of its
+// 268 MB, 82 % of the measured copy) and the y sweep 267 (69 %, 4.6 TB/s with
 // its close), against 384 and 390 before the slopes, face states and sums went through
 // pairs of components, minmod took three instructions, one reciprocal served
 // both star quotients, the physicality tests were made on the smallest values
 // and the options were fixed at compile time: x 66.2 -> 49.8 us, y 80.4 ->
-// 63.9 us a sweep, 57.8 since close_steps closes the steps.  Allaire at
-// 2048x1024: x 62.7 -> 45.9 us, y 84.8 -> 68.1, then 60.0 us
+// 63.9 us a sweep, 57.9 since close_steps closes the steps.  Allaire at
+// 2048x1024: x 62.7 -> 45.9 us, then 44.7, y 84.8 -> 68.1, then 60.9 us
 // (x with its rows staged and 5 CTAs per SM instead of the next row in
 // registers and 4: 49.1 -> 45.9).
 template <int MODEL, int OPT>
