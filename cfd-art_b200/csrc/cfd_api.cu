@@ -885,36 +885,51 @@ int cfd_upload(cfd_solver* s, const double* host, int layout, int n, double t) {
     return CFD_OK;
 }
 
-// Whether `bytes` from `p` on are this device's own memory, of one allocation.
-// Memory mapped in pieces counts as one allocation a piece.
+static void* driver_entry(const char* name) {
+    void* f = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPoint(name, &f, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+        f = nullptr;
+    cudaGetLastError();
+    return f;
+}
+
+// Whether `bytes` from `p` on are this device's own memory, of one allocation
+// or of mapped pieces that follow one another (neither of cudaMalloc, which IPC
+// handles take, nor of a pool, so no allocation's end lies between them).
 static bool own_range(const void* p, size_t bytes) {
     using Range = CUresult (*)(CUdeviceptr*, size_t*, CUdeviceptr);
-    static const Range range = [] {
-        void* f = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuMemGetAddressRange", &f, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess)
-            f = nullptr;
-        cudaGetLastError();
-        return reinterpret_cast<Range>(f);
-    }();
-    cudaPointerAttributes pa = {};
+    using Attribute = CUresult (*)(void*, CUpointer_attribute, CUdeviceptr);
+    static const auto range = reinterpret_cast<Range>(driver_entry("cuMemGetAddressRange"));
+    static const auto attribute = reinterpret_cast<Attribute>(driver_entry("cuPointerGetAttribute"));
     int device = -1;
-    const bool here = cudaGetDevice(&device) == cudaSuccess &&
-                      cudaPointerGetAttributes(&pa, p) == cudaSuccess &&
-                      pa.type == cudaMemoryTypeDevice && pa.device == device;
-    cudaGetLastError();
-    CUdeviceptr base = 0;
-    size_t size = 0;
-    const CUdeviceptr a = (CUdeviceptr)(uintptr_t)p;
-    return here && range && range(&base, &size, a) == CUDA_SUCCESS && a + bytes <= base + size;
+    if (!range || !attribute || cudaGetDevice(&device) != cudaSuccess) return false;
+    for (CUdeviceptr a = (CUdeviceptr)(uintptr_t)p;;) {
+        cudaPointerAttributes pa = {};
+        const bool here = cudaPointerGetAttributes(&pa, (const void*)(uintptr_t)a) == cudaSuccess &&
+                          pa.type == cudaMemoryTypeDevice && pa.device == device;
+        cudaGetLastError();
+        CUdeviceptr base = 0;
+        size_t size = 0;
+        if (!here || range(&base, &size, a) != CUDA_SUCCESS) return false;
+        const size_t n = base + size - a;
+        if (n >= bytes) return true;
+        int ipc = 1;
+        CUmemoryPool pool = nullptr;
+        if (attribute(&ipc, CU_POINTER_ATTRIBUTE_IS_LEGACY_CUDA_IPC_CAPABLE, a) != CUDA_SUCCESS || ipc ||
+            attribute(&pool, CU_POINTER_ATTRIBUTE_MEMPOOL_HANDLE, a) != CUDA_SUCCESS || pool)
+            return false;
+        a += n;
+        bytes -= n;
+    }
 }
 
 int cfd_upload_device(cfd_solver* s, const double* dev, int n, double t) {
     if (!s || !dev) return fail(CFD_ERR_INVALID, "null argument");
     const cfd_config& c = s->cfg;
     int r;
-    // planes within an allocation of this device are read by the kernel, anything
+    // planes within this device's memory (own_range) are read by the kernel, anything
     // else that a copy takes (another device's memory, the host's, unaligned or the
     // solver's own planes) is copied, and what a copy refuses (planes that go
     // past their allocation) is refused by it

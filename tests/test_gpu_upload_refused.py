@@ -2,11 +2,15 @@
 are larger than the allocation they lie in, which the driver's copies refuse.
 (The next allocation follows it directly, so the memory past its end exists.)"""
 import ctypes
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
 
 import cfdgpu as G
+from cfdtest import ROOT
 
 pytestmark = pytest.mark.gpu
 
@@ -52,3 +56,33 @@ def test_refused_upload_changes_nothing(offset, steps):
             s.advance(3)
             untouched.advance(3)
             assert np.array_equal(s.download(), untouched.download())
+
+
+SEGMENTS = r"""
+import sys
+sys.path.insert(0, sys.argv[1])
+import numpy as np, torch
+import cfdgpu as G
+cfg = G.recipe_config("shock_bubbles", 1500, 1100)
+ic = G.recipe_ic(cfg, "shock_bubbles", nbubbles=4)
+planes = np.ascontiguousarray(ic[2:-2, 2:-2].transpose(2, 0, 1))
+dev = torch.from_numpy(planes).cuda()
+torch.cuda.synchronize()
+out = []
+for put in (lambda s: s.upload_device(dev.data_ptr()), lambda s: s.upload(planes, layout=G.SOA)):
+    with G.Solver(cfg) as s:
+        put(s)
+        s.advance(2)
+        out.append(s.download().tobytes())
+assert out[0] == out[1]
+print("same")
+"""
+
+
+def test_planes_in_mapped_pieces():
+    """53 MB of an allocator that maps its memory in pieces."""
+    pytest.importorskip("torch")
+    env = dict(os.environ, PYTORCH_CUDA_ALLOC_CONF="expandable_segments:True")
+    out = subprocess.run([sys.executable, "-c", SEGMENTS, str(ROOT / "cfd-art_b200")], capture_output=True,
+                         text=True, timeout=300, env=env)
+    assert out.returncode == 0 and out.stdout.strip() == "same", out.stderr[-2000:]
